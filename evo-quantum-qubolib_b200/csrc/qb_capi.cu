@@ -1376,8 +1376,8 @@ int batch_run(qb_handle* h, const qb_problem* problems, const std::vector<int32_
     P.n_max = n_tc_max;
     P.err = tc_err;
     const qb::TcSmemLayout L = qb::tc_layout(n_tc_max);
-    if (tc_pair) {  // plus the second tile's row terms of each B stage
-      sm_tc = std::max<size_t>(L.total + qb::kTcBStages * 128 * 4, 120 * 1024) + 1024;
+    if (tc_pair) {
+      sm_tc = qb::tc2_smem_bytes(n_tc_max);
       QB_CUDA(cudaFuncSetAttribute(qb::tc_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_tc));
     } else {
       sm_tc = std::max<size_t>(L.total, 120 * 1024) + 1024;
@@ -1417,7 +1417,7 @@ int batch_run(qb_handle* h, const qb_problem* problems, const std::vector<int32_
         qb::Tc2Params Q2{};
         Q2.P = P;
         Q2.tabs = static_cast<const qb::Tc2Tab*>(B[14].p);
-        qb::tc_pair_kernel<true><<<(unsigned)(first.size() - 1), qb::kTcThreads, sm_tc, st>>>(Q2);
+        qb::tc_pair_kernel<true><<<(unsigned)(first.size() - 1), qb::kTc2Threads, sm_tc, st>>>(Q2);
       } else
         qb::tc_pass1_kernel<true><<<(unsigned)(first.size() - 1), qb::kTcThreads, sm_tc, st>>>(P);
       ++h->kernels;
