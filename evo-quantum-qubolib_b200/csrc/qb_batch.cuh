@@ -51,27 +51,6 @@ struct BatchCand {  // a record to evaluate exactly
   uint64_t rid;
 };
 
-__host__ __device__ __forceinline__ uint64_t ord_f64(double e) {
-#ifdef __CUDA_ARCH__
-  uint64_t u = (uint64_t)__double_as_longlong(e);
-#else
-  uint64_t u;
-  memcpy(&u, &e, 8);
-#endif
-  return (u >> 63) ? ~u : (u | 0x8000000000000000ull);
-}
-
-__host__ __device__ __forceinline__ double unord_f64(uint64_t k) {
-  uint64_t u = (k >> 63) ? (k & 0x7fffffffffffffffull) : ~k;
-#ifdef __CUDA_ARCH__
-  return __longlong_as_double((long long)u);
-#else
-  double e;
-  memcpy(&e, &u, 8);
-  return e;
-#endif
-}
-
 __device__ __forceinline__ ProblemDev batch_problem(const BatchInst& I, const double* W) {
   return ProblemDev{I.n, W + I.w_off};
 }
@@ -172,11 +151,11 @@ __global__ void batch_select_kernel(const BatchInst* __restrict__ insts, const u
 }
 
 // 4. exact evaluation of candidate s = blockIdx.x (s < min(count, cap))
-__global__ void __launch_bounds__(kExactThreads)
+__global__ void __launch_bounds__(kExactThreads, 2)
 batch_exact_kernel(const BatchInst* __restrict__ insts, const double* __restrict__ W,
                    const BatchCand* __restrict__ cand, const int* __restrict__ cand_count, int cap,
                    ExactOut* __restrict__ out, uint64_t* __restrict__ emin) {
-  extern __shared__ double bex_smem[];
+  extern __shared__ __align__(16) double bex_smem[];
   const int count = min(*cand_count, cap);
   if ((int)blockIdx.x >= count) return;
   const BatchCand c = cand[blockIdx.x];

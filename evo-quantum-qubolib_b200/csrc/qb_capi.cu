@@ -1623,22 +1623,34 @@ int qb_prefix_minima(qb_handle* h, const qb_problem* p, int32_t prefix_bits, dou
   qb::TieRule rule{qb::kTieNatural, n, 0, 0, 0};
   const qb::ProblemDev pd{n, static_cast<const double*>(h->W.p)};
   const uint64_t count = 1ull << A;
-  QB_CUDA(h->exout.ensure(count * sizeof(qb::ExactOut)));
+  // few prefixes: each split over 2^sb CTAs (of at least 2^14 states) as long as all of them run
+  // at once, two per SM; more CTAs repeat the set-up, fewer leave SMs idle.  Measured for the
+  // whole call (us) at sb = 0 1 2 3 4 5: n = 27, A = 7 182 128 132 149 167 221; n = 24, A = 4
+  // 177 113 77 56 52 58; n = 23, A = 3 176 112 77 55 52 43; n = 30, A = 10 683 672 738 864
+  int sb = 0;
+  while (sb < B - 14 && (count << (sb + 1)) <= 2ull * (uint64_t)h->sm_count) ++sb;
+  const uint64_t nout = count << sb;
+  QB_CUDA(h->exout.ensure(nout * sizeof(qb::ExactOut)));
   const size_t sm = qb::exact_smem_bytes(n, B);
   QB_CUDA(cudaFuncSetAttribute(qb::exact_records_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-  const uint64_t maxg = 1u << 30;
+  const uint64_t maxg = 1u << 30;  // sb > 0 only far below it
   for (uint64_t off = 0; off < count; off += maxg) {
     const uint64_t g = std::min<uint64_t>(maxg, count - off);
-    qb::exact_records_kernel<<<(unsigned)g, qb::kExactThreads, sm, h->st>>>(
-        pd, rule, geom, nullptr, nullptr, (int64_t)count, (int64_t)off, static_cast<qb::ExactOut*>(h->exout.p) + off, 0);
+    qb::exact_records_kernel<<<(unsigned)(g << sb), qb::kExactThreads, sm, h->st>>>(
+        pd, rule, geom, nullptr, nullptr, (int64_t)count, (int64_t)off, static_cast<qb::ExactOut*>(h->exout.p) + off, sb);
     ++h->kernels;
   }
   QB_CUDA(cudaGetLastError());
-  QB_CUDA(h->hout.ensure(count * sizeof(qb::ExactOut)));
-  QB_CUDA(cudaMemcpyAsync(h->hout.p, h->exout.p, count * sizeof(qb::ExactOut), cudaMemcpyDeviceToHost, h->st));
+  QB_CUDA(h->hout.ensure(nout * sizeof(qb::ExactOut)));
+  QB_CUDA(cudaMemcpyAsync(h->hout.p, h->exout.p, nout * sizeof(qb::ExactOut), cudaMemcpyDeviceToHost, h->st));
   QB_CUDA(cudaStreamSynchronize(h->st));
   const qb::ExactOut* eo = static_cast<const qb::ExactOut*>(h->hout.p);
-  for (uint64_t i = 0; i < count; ++i) out[i] = eo[qb::gray64(i)].e;  // QBF's prefix visiting order
+  for (uint64_t i = 0; i < count; ++i) {  // QBF's prefix visiting order
+    const qb::ExactOut* r = eo + (qb::gray64(i) << sb);
+    double e = r[0].e;
+    for (int q = 1; q < (1 << sb); ++q) e = std::min(e, r[q].e);
+    out[i] = e;
+  }
   return QB_OK;
 }
 
