@@ -913,7 +913,8 @@ int qbf1_wrap_solve(qb_handle* h, const qb_problem* p, const qb_options* o, qb_r
   QB_CUDA(B[6].ensure(cols * sizeof(short)));
   QB_CUDA(B[7].ensure((size_t)A * cols * sizeof(short)));
   QB_CUDA(B[8].ensure(steps * sizeof(short)));
-  QB_CUDA(B[9].ensure((qb::kQbf1Threads + 1) * sizeof(unsigned long long)));
+  constexpr size_t key_bytes = qb::kQbf1Threads * sizeof(unsigned long long);
+  QB_CUDA(B[9].ensure(key_bytes + sizeof(qb::Qbf1Answer)));
   QB_CUDA(cudaMemcpyAsync(B[0].p, Qi.data(), Qi.size() * sizeof(int), cudaMemcpyHostToDevice, h->st));
   h->h2d += (int64_t)(Qi.size() * sizeof(int));
   const int* dQ = static_cast<const int*>(B[0].p);
@@ -921,9 +922,11 @@ int qbf1_wrap_solve(qb_handle* h, const qb_problem* p, const qb_options* o, qb_r
   short* ABBA = static_cast<short*>(B[7].p);
   short* AA = static_cast<short*>(B[8].p);
   unsigned long long* key = static_cast<unsigned long long*>(B[9].p);
-  QB_CUDA(cudaMemsetAsync(key, 0xff, (qb::kQbf1Threads + 1) * sizeof(unsigned long long), h->st));
+  qb::Qbf1Answer* ans = reinterpret_cast<qb::Qbf1Answer*>(key + qb::kQbf1Threads);
+  QB_CUDA(cudaMemsetAsync(key, 0xff, key_bytes + sizeof(qb::Qbf1Answer), h->st));
   QB_CUDA(cudaEventRecord(h->ev[0], h->st));
-  qb::qbf1w_tables_kernel<<<(unsigned)(cols / 256), 256, (size_t)n * n * sizeof(int), h->st>>>(dQ, n, A, BB, ABBA);
+  const size_t smt = qb::qbf1w_tables_smem(n, A);
+  qb::qbf1w_tables_kernel<<<1u << (qb::kQbf1B - qb::kQbf1Lo), 256, smt, h->st>>>(dQ, n, A, BB, ABBA);
   qb::qbf1w_prefix_kernel<<<(unsigned)std::min<uint64_t>((steps + 255) / 256, (uint64_t)h->sm_count * 8), 256,
                             (size_t)A * A * sizeof(int), h->st>>>(dQ, n, A, AA);
   const uint64_t nchunks = std::min<uint64_t>(64, std::max<uint64_t>(4, steps));
@@ -934,30 +937,22 @@ int qbf1_wrap_solve(qb_handle* h, const qb_problem* p, const qb_options* o, qb_r
   qb::qbf1w_search_kernel<<<dim3(qb::kQbf1Threads / 64, (unsigned)(nchunks / 4)), 256, sm, h->st>>>(
       A, BB, ABBA, AA, chunk_len, key);
   QB_CUDA(cudaEventRecord(h->ev[5], h->st));
-  h->kernels += 3;
-  QB_CUDA(cudaGetLastError());
-  QB_CUDA(h->hout.ensure(qb::kQbf1Threads * sizeof(unsigned long long)));
-  QB_CUDA(cudaMemcpyAsync(h->hout.p, key, qb::kQbf1Threads * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                          h->st));
-  h->d2h += (int64_t)qb::kQbf1Threads * 8;
-  QB_CUDA(cudaStreamSynchronize(h->st));
-  // the host's argmin over the threads' best values: the lowest thread among equals
-  const unsigned long long* hk = static_cast<const unsigned long long*>(h->hout.p);
-  int tid = 0;
-  for (int i = 1; i < qb::kQbf1Threads; ++i)
-    if ((hk[i] >> 40) < (hk[tid] >> 40)) tid = i;
-  if (hk[tid] == ~0ull) return QB_ECUDA;
-  const int best16 = (int)(hk[tid] >> 40) - 32768;
-  const uint64_t step = hk[tid] & ((1ull << 40) - 1);
-  const uint64_t prefix = qb::gray64(step);
-  qb::qbf1w_row_kernel<<<(unsigned)(cols / 256), 256, 0, h->st>>>(A, BB, ABBA, prefix, key + qb::kQbf1Threads);
-  ++h->kernels;
+  // the winning thread, its exact step and that prefix's suffix, then one copy back
+  qb::qbf1w_final_kernel<<<1, 512, 0, h->st>>>(A, BB, ABBA, AA, key, qb::qbf1w_group(chunk_len), ans);
+  qb::qbf1w_row_kernel<<<(unsigned)(cols / 256), 256, 0, h->st>>>(A, BB, ABBA, ans);
+  h->kernels += 5;
   QB_CUDA(cudaGetLastError());
   QB_CUDA(cudaEventRecord(h->ev[1], h->st));
-  QB_CUDA(cudaMemcpyAsync(h->hmisc.p, key + qb::kQbf1Threads, 8, cudaMemcpyDeviceToHost, h->st));
-  h->d2h += 8;
+  static_assert(sizeof(qb::Qbf1Answer) <= 64, "hmisc");
+  QB_CUDA(cudaMemcpyAsync(h->hmisc.p, ans, sizeof(qb::Qbf1Answer), cudaMemcpyDeviceToHost, h->st));
+  h->d2h += (int64_t)sizeof(qb::Qbf1Answer);
   QB_CUDA(cudaStreamSynchronize(h->st));
-  const uint64_t sfx = *static_cast<const unsigned long long*>(h->hmisc.p) & 0xffffffffull;
+  const qb::Qbf1Answer ha = *static_cast<const qb::Qbf1Answer*>(h->hmisc.p);
+  if (ha.found != 1) return QB_ECUDA;
+  const int tid = ha.tid, best16 = ha.best16;
+  const uint64_t step = ha.step;
+  const uint64_t prefix = qb::gray64(step);
+  const uint64_t sfx = ha.row & 0xffffffffull;
   const uint64_t X = (prefix << qb::kQbf1B) | sfx;
   double e = 0.0;  // exact energy of the reported state
   for (int i = 0; i < n; ++i) {
