@@ -119,17 +119,22 @@ struct qb_handle_s {
   int device = 0;
   cudaStream_t own = nullptr;
   cudaStream_t st = nullptr;
-  DevBuf W, gtab, rec, cand, misc, exout, tcscratch;
+  DevBuf W;  // SolveCtl, W (n*n doubles), W times the tensor-core plan's scale (n*n doubles)
+  DevBuf gtab, rec, cand, misc, exout;
   DevBuf bat[15];  // qb_solve_batch: W, insts, gtab items, unit items, selection ids, cands, out, G tables,
                    // records, minima, scaled W, tensor-core items, item ranges, error word
-  HostBuf hW, hmisc, hout, hbat;  // hbat: qb_solve_batch's packed W matrices (pinned)
+  HostBuf hW, hmisc, hout, hbat;  // hW: the upload of W; hbat: qb_solve_batch's packed W matrices (pinned)
+  HostBuf hraw;                    // a device matrix copied back (pinned)
   HostBuf hstage;                  // qb_solve_batch: descriptors and work lists (pinned)
   // qb_solve_batch with QB_FLAG_GRAPH: the captured launch sequence of the last batch and
   // the fingerprint (shapes, options, buffer addresses) it is valid for
   cudaGraphExec_t batch_graph = nullptr;
   std::vector<uint64_t> batch_graph_key;
   int batch_graph_kernels = 0;
-  cudaEvent_t ev[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};  // 4, 5: main kernel
+  // 0 start, 1 end of pass 1, 2, 3 pass 2, 4, 5 main kernel; main0: the event at the main kernel's
+  // start (0 where nothing runs before it)
+  cudaEvent_t ev[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+  int main0 = 4;
   int64_t h2d = 0, d2h = 0;  // bytes copied by the current call
   float kernel_ms = 0.f;
   int sm_count = 0;
@@ -176,17 +181,6 @@ int dtype_size(int dt) {
   }
 }
 
-double load_elem(const unsigned char* p, int dt) {
-  switch (dt) {
-    case QB_F32: { float v; memcpy(&v, p, 4); return v; }
-    case QB_F64: { double v; memcpy(&v, p, 8); return v; }
-    case QB_I8: { int8_t v; memcpy(&v, p, 1); return v; }
-    case QB_I16: { int16_t v; memcpy(&v, p, 2); return v; }
-    case QB_I32: { int32_t v; memcpy(&v, p, 4); return v; }
-    default: { int64_t v; memcpy(&v, p, 8); return (double)v; }
-  }
-}
-
 template <class T>
 int host_problem_typed(const qb_problem* p, double* Wout, double* abs_sum) {
   const int n = p->n;
@@ -230,31 +224,19 @@ int load_host_problem_into(const qb_problem* p, double* Wout, double* abs_sum, b
 // Q (any dtype, host or device) -> W (n x n doubles) and sum |Q_ij|.
 int load_problem(qb_handle* h, const qb_problem* p, std::vector<double>& W, double* abs_sum, bool* is_int) {
   const int n = p->n;
+  W.resize((size_t)n * n);
+  if (!p->q_on_device) return load_host_problem_into(p, W.data(), abs_sum, is_int);
   const int es = dtype_size(p->dtype);
-  std::vector<unsigned char> raw((size_t)n * n * es);
-  if (p->q_on_device) {
-    QB_CUDA(cudaMemcpy2DAsync(raw.data(), (size_t)n * es, p->q, (size_t)p->ldq * es, (size_t)n * es, n,
-                              cudaMemcpyDeviceToHost, h->st));
-    QB_CUDA(cudaStreamSynchronize(h->st));
-    h->d2h += (int64_t)n * n * es;
-  } else {
-    const unsigned char* src = static_cast<const unsigned char*>(p->q);
-    for (int i = 0; i < n; ++i) memcpy(raw.data() + (size_t)i * n * es, src + (size_t)i * p->ldq * es, (size_t)n * es);
-  }
-  *is_int = p->dtype >= QB_I8;
-  W.assign((size_t)n * n, 0.0);
-  double s = 0.0;
-  std::vector<double> Q((size_t)n * n);
-  for (size_t i = 0; i < Q.size(); ++i) {
-    double v = load_elem(raw.data() + i * es, p->dtype);
-    if (!std::isfinite(v)) return QB_EINVAL;
-    Q[i] = v;
-    s += std::fabs(v);
-  }
-  for (int i = 0; i < n; ++i)
-    for (int j = 0; j < n; ++j) W[(size_t)i * n + j] = (i == j) ? Q[(size_t)i * n + i] : Q[(size_t)i * n + j] + Q[(size_t)j * n + i];
-  *abs_sum = s;
-  return QB_OK;
+  QB_CUDA(h->hraw.ensure((size_t)n * n * es));
+  QB_CUDA(cudaMemcpy2DAsync(h->hraw.p, (size_t)n * es, p->q, (size_t)p->ldq * es, (size_t)n * es, n,
+                            cudaMemcpyDeviceToHost, h->st));
+  QB_CUDA(cudaStreamSynchronize(h->st));
+  h->d2h += (int64_t)n * n * es;
+  qb_problem host = *p;
+  host.q = h->hraw.p;
+  host.ldq = n;
+  host.q_on_device = 0;
+  return load_host_problem_into(&host, W.data(), abs_sum, is_int);
 }
 
 int make_rule(const qb_options* o, int n, qb::TieRule* r) {
@@ -383,22 +365,37 @@ void fill_plan_fields(const qb_handle* h, const Plan& P, qb_result* r) {
   r->tc_kernel = P.form != QB_FORM_TC ? 0 : (P.tc.pair ? (P.tc.u16 ? 4 : 2) : (P.tc.u16 ? 3 : 1));
 }
 
-int upload_W(qb_handle* h, const std::vector<double>& W) {
-  size_t bytes = W.size() * sizeof(double);
+constexpr size_t kCtlBytes = 128;  // SolveCtl's room before W
+static_assert(sizeof(qb::SolveCtl) <= kCtlBytes, "control block");
+
+qb::SolveCtl* dev_ctl(qb_handle* h) { return static_cast<qb::SolveCtl*>(h->W.p); }
+const double* dev_W(qb_handle* h) { return reinterpret_cast<const double*>(static_cast<char*>(h->W.p) + kCtlBytes); }
+
+// One copy: the control block at its initial values, W and, with scale != 0, W times scale
+// behind it.
+int upload_W(qb_handle* h, const std::vector<double>& W, double scale = 0.0) {
+  const size_t nn = W.size();
+  const size_t bytes = kCtlBytes + (scale != 0.0 ? 2 : 1) * nn * sizeof(double);
   QB_CUDA(h->hW.ensure(bytes));
-  QB_CUDA(h->W.ensure(bytes));
-  memcpy(h->hW.p, W.data(), bytes);
+  QB_CUDA(h->W.ensure(kCtlBytes + 2 * nn * sizeof(double)));
+  qb::SolveCtl c{};
+  c.min_key = 0xffffffffu;
+  memcpy(h->hW.p, &c, sizeof(c));
+  double* dst = reinterpret_cast<double*>(static_cast<char*>(h->hW.p) + kCtlBytes);
+  memcpy(dst, W.data(), nn * sizeof(double));
+  if (scale != 0.0)
+    for (size_t i = 0; i < nn; ++i) dst[nn + i] = W[i] * scale;
   QB_CUDA(cudaMemcpyAsync(h->W.p, h->hW.p, bytes, cudaMemcpyHostToDevice, h->st));
   h->h2d += (int64_t)bytes;
   return QB_OK;
 }
 
 int run_pass1(qb_handle* h, Plan& P) {
-  const qb::ProblemDev pd{P.n, static_cast<const double*>(h->W.p)};
+  const qb::ProblemDev pd{P.n, dev_W(h)};
+  h->main0 = 4;
   if (P.form == QB_FORM_EXACT) {
     QB_CUDA(h->exout.ensure(std::max<uint64_t>(P.rec_count, 1) * sizeof(qb::ExactOut)));
     size_t sm = qb::exact_smem_bytes(P.n, P.geom.fbits);
-    QB_CUDA(cudaFuncSetAttribute(qb::exact_records_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     // chunked over the grid limit
     const uint64_t maxg = 1u << 30;
     QB_CUDA(cudaEventRecord(h->ev[4], h->st));
@@ -417,7 +414,6 @@ int run_pass1(qb_handle* h, Plan& P) {
   if (P.form == QB_FORM_GRAY) {
     QB_CUDA(h->gtab.ensure(((size_t)1 << P.a) * 32 * sizeof(float)));
     size_t sm0 = qb::gray_gtab_smem(P.n, P.a);
-    QB_CUDA(cudaFuncSetAttribute(qb::gray_gtab_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm0));
     unsigned gblocks = (unsigned)std::min<uint64_t>((1ull << P.a) / 8 + 1, (uint64_t)h->sm_count * 4);
     qb::gray_gtab_kernel<<<gblocks, 256, sm0, h->st>>>(pd, P.a, P.b, static_cast<float*>(h->gtab.p));
     ++h->kernels;
@@ -432,7 +428,6 @@ int run_pass1(qb_handle* h, Plan& P) {
     gp.gtab = static_cast<const float*>(h->gtab.p);
     gp.rec = static_cast<float*>(h->rec.p);
     size_t sm = qb::gray_pass1_smem(P.n, P.a);
-    QB_CUDA(cudaFuncSetAttribute(qb::gray_pass1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     uint64_t units = P.unit_end - P.unit_begin;
     QB_CUDA(cudaEventRecord(h->ev[4], h->st));
     if (units) {
@@ -443,16 +438,48 @@ int run_pass1(qb_handle* h, Plan& P) {
     QB_CUDA(cudaGetLastError());
     return QB_OK;
   }
-  QB_CUDA(h->tcscratch.ensure(qb::tc_scratch_bytes(P.tc)));
-  int rc = qb::tc_prepare(P.tc, pd, h->tcscratch.p, h->st, &h->kernels);
-  if (rc) return rc;
-  QB_CUDA(cudaEventRecord(h->ev[4], h->st));
-  rc = P.tc.pair ? qb::tc2_launch(P.tc, P.tc.gamma, static_cast<float*>(h->rec.p), h->tcscratch.p, h->st,
-                                  h->sm_count, &h->kernels)
-                 : qb::tc_launch(P.tc, static_cast<float*>(h->rec.p), h->tcscratch.p, h->st, h->sm_count, &h->kernels);
+  h->main0 = 0;  // nothing before the search kernel
+  unsigned* err = &dev_ctl(h)->err;
+  const double* Wsc = dev_W(h) + (size_t)P.n * P.n;
+  const int rc = P.tc.pair ? qb::tc2_launch(P.tc, P.tc.gamma, static_cast<float*>(h->rec.p), Wsc, err,
+                                            &dev_ctl(h)->min_key, h->st, h->sm_count, &h->kernels)
+                           : qb::tc_launch(P.tc, static_cast<float*>(h->rec.p), Wsc, err, h->st, h->sm_count, &h->kernels);
   if (rc) return rc;
   QB_CUDA(cudaEventRecord(h->ev[5], h->st));
   return QB_OK;
+}
+
+// Lets a kernel use all of an SM's shared memory (the launches ask for what they need): once
+// per handle instead of before every launch.
+template <class K>
+cudaError_t allow_shared(K* kern) {
+  cudaFuncAttributes a{};
+  const cudaError_t e = cudaFuncGetAttributes(&a, kern);
+  if (e != cudaSuccess) return e;
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - (int)a.sharedSizeBytes);
+}
+
+cudaError_t allow_shared_all() {
+  cudaError_t e = cudaSuccess;
+  auto add = [&](auto* k) {
+    if (e == cudaSuccess) e = allow_shared(k);
+  };
+  add(qb::exact_records_kernel);
+  add(qb::exact_candidates_kernel);
+  add(qb::exact_row_kernel);
+  add(qb::gray_gtab_kernel);
+  add(qb::gray_pass1_kernel);
+  add(qb::tc_pass1_kernel<false, false>);
+  add(qb::tc_pass1_kernel<false, true>);
+  add(qb::tc_pass1_kernel<true>);
+  add(qb::tc_pair_fp32_kernel);
+  add(qb::tc_pair_kernel<false>);
+  add(qb::tc_pair_kernel<true>);
+  add(qb::batch_gtab_kernel);
+  add(qb::batch_gray_kernel);
+  add(qb::batch_exact_kernel);
+  add(qb::qbf1w_search_kernel);
+  return e;
 }
 
 }  // namespace
@@ -491,6 +518,7 @@ int qb_handle_create(int device, qb_handle** out) {
   cudaError_t e = cudaStreamCreateWithFlags(&h->own, cudaStreamNonBlocking);
   for (int i = 0; i < 6 && e == cudaSuccess; ++i) e = cudaEventCreate(&h->ev[i]);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&h->sm_count, cudaDevAttrMultiProcessorCount, device);
+  if (e == cudaSuccess) e = allow_shared_all();
   if (e != cudaSuccess) {
     qb_handle_destroy(h);
     return cuda_fail(e);
@@ -510,13 +538,13 @@ int qb_handle_destroy(qb_handle* h) {
   h->cand.release();
   h->misc.release();
   h->exout.release();
-  h->tcscratch.release();
   for (auto& b : h->bat) b.release();
   h->hW.release();
   h->hmisc.release();
   h->hout.release();
   h->hbat.release();
   h->hstage.release();
+  h->hraw.release();
   if (h->batch_graph) cudaGraphExecDestroy(h->batch_graph);
   for (auto& ev : h->ev)
     if (ev) cudaEventDestroy(ev);
@@ -530,7 +558,8 @@ int qb_handle_destroy(qb_handle* h) {
 namespace {
 
 // validation, problem upload and the pass-1 launch of qb_solve_begin
-int begin_launch(qb_handle* h, const qb_problem* p, const qb_options* o, Plan& P) {
+// (fused: qb_solve's whole-problem path, whose exact form has no pass 1)
+int begin_launch(qb_handle* h, const qb_problem* p, const qb_options* o, Plan& P, bool fused) {
   if (p->n < 1 || p->n > qb::kMaxN || !p->q || p->ldq < p->n || dtype_size(p->dtype) == 0) return QB_EINVAL;
   if (o->shard_count > 1 && (o->shard_index < 0 || o->shard_index >= o->shard_count)) return QB_EINVAL;
   QB_CUDA(cudaSetDevice(h->device));
@@ -573,10 +602,11 @@ int begin_launch(qb_handle* h, const qb_problem* p, const qb_options* o, Plan& P
                  (P.tc.pair ? qb::tc2_u16_eligible(P.n, W.data(), &P.tc.dmin) : qb::tc_u16_eligible(P.n, W.data(), &P.tc.dmin));
     }
   }
-  rc = upload_W(h, W);
+  rc = upload_W(h, W, P.form == QB_FORM_TC ? P.tc.scale : 0.0);
   if (rc) return rc;
   QB_CUDA(h->misc.ensure(64));
   QB_CUDA(h->hmisc.ensure(64));
+  if (fused && P.form == QB_FORM_EXACT) return QB_OK;
   QB_CUDA(cudaEventRecord(h->ev[0], h->st));
   return run_pass1(h, P);
 }
@@ -608,15 +638,17 @@ int begin_finish_pass1(qb_handle* h, Plan& P, double* local_min) {
     h->d2h += (int64_t)sizeof(uint32_t);
     QB_CUDA(cudaStreamSynchronize(h->st));
     if (P.form == QB_FORM_TC) {
-      int trc = qb::tc_check_error(h->tcscratch.p, h->st);
+      unsigned e = 0;
+      QB_CUDA(cudaMemcpyAsync(&e, &dev_ctl(h)->err, sizeof(unsigned), cudaMemcpyDeviceToHost, h->st));
+      QB_CUDA(cudaStreamSynchronize(h->st));
       h->d2h += (int64_t)sizeof(unsigned);
-      if (trc) return trc;
+      if (e & qb::kErrTimeout) return QB_ETIMEOUT;
     }
     uint32_t key = *static_cast<uint32_t*>(h->hmisc.p);
     lmin = (P.rec_count && key != 0xffffffffu) ? (double)qb::key2f(key) : INFINITY;
   }
   QB_CUDA(cudaEventElapsedTime(&h->pass1_ms, h->ev[0], h->ev[1]));
-  QB_CUDA(cudaEventElapsedTime(&h->kernel_ms, h->ev[4], h->ev[5]));
+  QB_CUDA(cudaEventElapsedTime(&h->kernel_ms, h->ev[h->main0], h->ev[5]));
   h->plan = P;
   h->local_min = lmin;
   h->pending = true;
@@ -624,33 +656,33 @@ int begin_finish_pass1(qb_handle* h, Plan& P, double* local_min) {
   return QB_OK;
 }
 
-// qb_solve of one whole problem (Gray or tensor-core form, QB_TIE_QBF / QB_TIE_NATURAL):
-// minimum, threshold, selection, exact re-evaluation and the final pick all on the device,
-// then one copy of the answer to the host.  Returns -1 when the candidates overflow the cap
-// (the caller then takes the two-phase path with a larger cap).
+// qb_solve of one whole problem: after pass 1 the minimum, the selection, the exact
+// re-evaluation and the final pick (with QB_F1's suffix step) follow on the device, then one copy
+// of the control block to the host.  The 16-bit pair kernel reduces its records' minimum itself,
+// so that a solve is three launches (four under QB_F1's rule): 65 us of device time against 107
+// at n = 20 .. 28 with the scaling, threshold and final kernels and the clears on their own, and
+// one host round trip against five under QB_F1's rule.  Returns -1 when the candidates overflow
+// the cap (the caller then takes the two-phase path with a larger cap).
 int solve_fused(qb_handle* h, const Plan& P, qb_result* r) {
-  char* m = static_cast<char*>(h->misc.p);  // [0] min key, [8] thr, [16] flag, [20] count, [24] best
-  uint32_t* mk = reinterpret_cast<uint32_t*>(m);
-  double* thr = reinterpret_cast<double*>(m + 8);
-  int* flag = reinterpret_cast<int*>(m + 16);
-  int* count = reinterpret_cast<int*>(m + 20);
-  qb::ExactOut* best = reinterpret_cast<qb::ExactOut*>(m + 24);
-  const unsigned* err = P.form == QB_FORM_TC ? static_cast<const unsigned*>(h->tcscratch.p) : nullptr;
-  QB_CUDA(cudaMemsetAsync(mk, 0xff, sizeof(uint32_t), h->st));
-  if (P.rec_count) {
+  qb::SolveCtl* ctl = dev_ctl(h);
+  const qb::ProblemDev pd{P.n, dev_W(h)};
+  const bool exact_form = P.form == QB_FORM_EXACT;
+  const bool min_done = P.form == QB_FORM_TC && P.tc.pair && P.tc.u16;
+  int pass1_end = 5;
+  if (!exact_form) {
     const unsigned blocks = (unsigned)std::min<uint64_t>((P.rec_count + 255) / 256, (uint64_t)h->sm_count * 8);
-    qb::rec_min_kernel<<<blocks, 256, 0, h->st>>>(static_cast<const float*>(h->rec.p), (int64_t)P.rec_count, mk);
-    ++h->kernels;
-  }
-  QB_CUDA(cudaEventRecord(h->ev[1], h->st));
-  QB_CUDA(cudaEventRecord(h->ev[2], h->st));
-  qb::rec_threshold_kernel<<<1, 1, 0, h->st>>>(mk, P.eps, P.is_int ? 1 : 0, err, thr, flag, count);
-  QB_CUDA(h->cand.ensure((size_t)h->cap * sizeof(uint64_t)));
-  if (P.rec_count) {
-    const unsigned blocks = (unsigned)std::min<uint64_t>((P.rec_count + 255) / 256, (uint64_t)h->sm_count * 8);
+    if (!min_done) {
+      qb::rec_min_kernel<<<blocks, 256, 0, h->st>>>(static_cast<const float*>(h->rec.p), (int64_t)P.rec_count,
+                                                    &ctl->min_key);
+      ++h->kernels;
+      QB_CUDA(cudaEventRecord(h->ev[1], h->st));
+      pass1_end = 1;
+    }
+    QB_CUDA(h->cand.ensure((size_t)h->cap * sizeof(uint64_t)));
     qb::rec_select_dev_kernel<<<blocks, 256, 0, h->st>>>(static_cast<const float*>(h->rec.p), (int64_t)P.rec_count,
-                                                         (int64_t)P.rec_begin, thr, flag,
-                                                         static_cast<uint64_t*>(h->cand.p), count, h->cap);
+                                                         (int64_t)P.rec_begin, ctl, P.eps, P.is_int ? 1 : 0,
+                                                         static_cast<uint64_t*>(h->cand.p), h->cap);
+    ++h->kernels;
   }
   int maxf = 0;
   {
@@ -659,45 +691,56 @@ int solve_fused(qb_handle* h, const Plan& P, qb_result* r) {
     maxf = __builtin_popcountll(f & qb::mask64(P.n));
   }
   if (maxf > qb::kExactMaxFree) return QB_EINVAL;
-  const int sb = std::max(0, std::min(4, maxf - 12));
-  QB_CUDA(h->exout.ensure(((size_t)h->cap << sb) * sizeof(qb::ExactOut)));
-  const qb::ProblemDev pd{P.n, static_cast<const double*>(h->W.p)};
-  const size_t sm = qb::exact_smem_bytes(P.n, maxf);
-  QB_CUDA(cudaFuncSetAttribute(qb::exact_candidates_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-  qb::exact_candidates_kernel<<<(unsigned)(2 * h->sm_count), qb::kExactThreads, sm, h->st>>>(
-      pd, P.rule, P.geom, static_cast<const uint64_t*>(h->cand.p), count, h->cap, sb,
-      static_cast<qb::ExactOut*>(h->exout.p));
-  qb::exact_final_kernel<<<1, 256, 0, h->st>>>(static_cast<const qb::ExactOut*>(h->exout.p), count, h->cap, sb, flag,
-                                               best);
-  h->kernels += 4;
+  const unsigned ctas = 2u * (unsigned)h->sm_count;
+  // parts of 2^13 states (no walked bits): at most 16 per candidate record, of which there are
+  // few; in the exact form as long as all CTAs run at once
+  int sb = std::max(0, std::min(4, maxf - 13));
+  if (exact_form)
+    while (sb > 0 && (P.rec_count << sb) > ctas) --sb;
+  QB_CUDA(h->exout.ensure((ctas + (1u << qb::kRowSplit)) * sizeof(qb::ExactOut)));
+  qb::ExactOut* part = static_cast<qb::ExactOut*>(h->exout.p);
+  if (exact_form) QB_CUDA(cudaEventRecord(h->ev[0], h->st));
+  const unsigned grid = exact_form ? (unsigned)std::min<uint64_t>(P.rec_count << sb, ctas) : ctas;
+  qb::exact_candidates_kernel<<<grid, qb::kExactThreads, qb::exact_smem_bytes(P.n, maxf), h->st>>>(
+      pd, P.rule, P.geom, exact_form ? nullptr : static_cast<const uint64_t*>(h->cand.p), ctl, (int64_t)P.rec_count,
+      h->cap, sb, part);
+  ++h->kernels;
+  if (exact_form) {
+    QB_CUDA(cudaEventRecord(h->ev[5], h->st));
+    h->main0 = 0;
+  }
+  if (P.rule.kind == qb::kTieQBF1) {
+    qb::exact_row_kernel<<<1u << qb::kRowSplit, qb::kExactThreads, qb::exact_smem_bytes(P.n, 18), h->st>>>(pd, ctl,
+                                                                                                        part + ctas);
+    ++h->kernels;
+  }
   QB_CUDA(cudaGetLastError());
   QB_CUDA(cudaEventRecord(h->ev[3], h->st));
-  QB_CUDA(cudaMemcpyAsync(h->hmisc.p, m, 48, cudaMemcpyDeviceToHost, h->st));
-  h->d2h += 48;
-  unsigned herr = 0;
-  if (err) {
-    QB_CUDA(cudaMemcpyAsync(&herr, err, sizeof(unsigned), cudaMemcpyDeviceToHost, h->st));
-    h->d2h += (int64_t)sizeof(unsigned);
-  }
+  QB_CUDA(cudaMemcpyAsync(h->hmisc.p, ctl, sizeof(qb::SolveCtl), cudaMemcpyDeviceToHost, h->st));
+  h->d2h += (int64_t)sizeof(qb::SolveCtl);
   QB_CUDA(cudaStreamSynchronize(h->st));
-  if (herr & qb::kErrTimeout) return QB_ETIMEOUT;
-  const char* hm = static_cast<const char*>(h->hmisc.p);
-  const uint32_t key = *reinterpret_cast<const uint32_t*>(hm);
-  const int zero = *reinterpret_cast<const int*>(hm + 16);
-  const int cnt = *reinterpret_cast<const int*>(hm + 20);
-  if (!zero && cnt > h->cap) return -1;
-  const qb::ExactOut b = *reinterpret_cast<const qb::ExactOut*>(hm + 24);
-  const bool found = zero ? (P.rec_begin == 0 && P.rec_count > 0) : cnt > 0;
+  const qb::SolveCtl c = *static_cast<const qb::SolveCtl*>(h->hmisc.p);
+  if (c.err & qb::kErrTimeout) return QB_ETIMEOUT;
+  if (!exact_form && c.count > h->cap) return -1;
+  double pass1_min = exact_form ? c.best.e : (c.min_key != 0xffffffffu ? (double)qb::key2f(c.min_key) : INFINITY);
+  // E(0) = 0 is minimal and X = 0 has the smallest key under every rule
+  const bool zero = !exact_form && P.is_int && P.eps == 0.0 && pass1_min >= 0.0;
+  qb::ExactOut b = zero ? qb::ExactOut{0.0, 0ull, 0ull} : c.best;
+  const bool found = zero || exact_form || c.count > 0;
+  if (found && P.rule.kind == qb::kTieQBF1 && b.x != 0) {
+    if (c.row.e != b.e) return QB_ECUDA;
+    b.x = c.row.x;
+  }
   memset(r, 0, sizeof(*r));
   r->form_used = P.form;
   r->is_integer = P.is_int ? 1 : 0;
-  r->pass1_min = (P.rec_count && key != 0xffffffffu) ? (double)qb::key2f(key) : INFINITY;
+  r->pass1_min = pass1_min;
   r->err_bound = P.eps;
   r->states = (int64_t)P.states;
-  r->candidate_records = zero ? 0 : cnt;
-  QB_CUDA(cudaEventElapsedTime(&r->pass1_ms, h->ev[0], h->ev[1]));
-  QB_CUDA(cudaEventElapsedTime(&r->pass2_ms, h->ev[2], h->ev[3]));
-  QB_CUDA(cudaEventElapsedTime(&r->kernel_ms, h->ev[4], h->ev[5]));
+  r->candidate_records = zero ? 0 : c.count;
+  QB_CUDA(cudaEventElapsedTime(&r->pass1_ms, h->ev[0], h->ev[pass1_end]));
+  QB_CUDA(cudaEventElapsedTime(&r->pass2_ms, h->ev[pass1_end], h->ev[3]));
+  QB_CUDA(cudaEventElapsedTime(&r->kernel_ms, h->ev[h->main0], h->ev[5]));
   r->found = found ? 1 : 0;
   r->best_x = b.x;
   r->best_e = found ? b.e : INFINITY;
@@ -718,7 +761,7 @@ extern "C" {
 int qb_solve_begin(qb_handle* h, const qb_problem* p, const qb_options* o, double* local_min) {
   if (!h || !p || !o || !local_min) return QB_EINVAL;
   Plan P;
-  int rc = begin_launch(h, p, o, P);
+  int rc = begin_launch(h, p, o, P, false);
   if (rc) return rc;
   return begin_finish_pass1(h, P, local_min);
 }
@@ -737,14 +780,13 @@ int rescore(qb_handle* h, const Plan& P, const qb::TieRule& rule, const qb::RecG
     maxf = __builtin_popcountll(f & qb::mask64(P.n));
   }
   if (maxf > qb::kExactMaxFree) return QB_EINVAL;
-  const qb::ProblemDev pd{P.n, static_cast<const double*>(h->W.p)};
+  const qb::ProblemDev pd{P.n, dev_W(h)};
   // few candidate records: split each over several CTAs (at least 2^12 states per CTA)
   int sb = 0;
   while (sb < maxf - 12 && ((int64_t)count << (sb + 1)) <= 2 * (int64_t)h->sm_count) ++sb;
   const size_t nout = (size_t)count << sb;
   QB_CUDA(h->exout.ensure(nout * sizeof(qb::ExactOut)));
   size_t sm = qb::exact_smem_bytes(P.n, maxf);
-  QB_CUDA(cudaFuncSetAttribute(qb::exact_records_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
   qb::exact_records_kernel<<<(unsigned)nout, qb::kExactThreads, sm, h->st>>>(
       pd, rule, geom, static_cast<const uint64_t*>(h->cand.p), nullptr, count, 0,
       static_cast<qb::ExactOut*>(h->exout.p), sb);
@@ -932,7 +974,6 @@ int qbf1_wrap_solve(qb_handle* h, const qb_problem* p, const qb_options* o, qb_r
   const uint64_t nchunks = std::min<uint64_t>(64, std::max<uint64_t>(4, steps));
   const uint64_t chunk_len = (steps + nchunks - 1) / nchunks;
   const size_t sm = qb::qbf1w_search_smem(A);
-  QB_CUDA(cudaFuncSetAttribute(qb::qbf1w_search_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
   QB_CUDA(cudaEventRecord(h->ev[4], h->st));
   qb::qbf1w_search_kernel<<<dim3(qb::kQbf1Threads / 64, (unsigned)(nchunks / 4)), 256, sm, h->st>>>(
       A, BB, ABBA, AA, chunk_len, key);
@@ -1000,13 +1041,14 @@ int qb_solve(qb_handle* h, const qb_problem* p, const qb_options* o, qb_result* 
     return QB_EINVAL;
   }
   Plan P;
-  int rc = begin_launch(h, p, o, P);
+  const bool whole = o->shard_count <= 1;
+  int rc = begin_launch(h, p, o, P, whole);
   if (rc) {
     memset(r, 0, sizeof(*r));
     r->status = rc;
     return rc;
   }
-  if (o->shard_count <= 1 && P.form != QB_FORM_EXACT && P.rule.kind != qb::kTieQBF1) {
+  if (whole) {
     rc = solve_fused(h, P, r);
     if (rc >= 0) {
       if (rc) {
@@ -1373,17 +1415,12 @@ int batch_run(qb_handle* h, const qb_problem* problems, const std::vector<int32_
     const qb::TcSmemLayout L = qb::tc_layout(n_tc_max);
     if (tc_pair) {
       sm_tc = qb::tc2_smem_bytes(n_tc_max);
-      QB_CUDA(cudaFuncSetAttribute(qb::tc_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_tc));
     } else {
       sm_tc = std::max<size_t>(L.total, 120 * 1024) + 1024;
-      QB_CUDA(cudaFuncSetAttribute(qb::tc_pass1_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_tc));
     }
   }
   if (any_gray) {
-    QB_CUDA(cudaFuncSetAttribute(qb::batch_gtab_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_gtab));
-    QB_CUDA(cudaFuncSetAttribute(qb::batch_gray_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_gray));
   }
-  QB_CUDA(cudaFuncSetAttribute(qb::batch_exact_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_exact));
   const unsigned key_blocks = (unsigned)std::min<int>((cap + 255) / 256, h->sm_count * 4);
 
   // the whole device side of the batch: uploads, the six launches, the result copy
@@ -1616,7 +1653,7 @@ int qb_prefix_minima(qb_handle* h, const qb_problem* p, int32_t prefix_bits, dou
   geom.n = n;
   geom.fbits = B;
   qb::TieRule rule{qb::kTieNatural, n, 0, 0, 0};
-  const qb::ProblemDev pd{n, static_cast<const double*>(h->W.p)};
+  const qb::ProblemDev pd{n, dev_W(h)};
   const uint64_t count = 1ull << A;
   // few prefixes: each split over 2^sb CTAs (of at least 2^14 states) as long as all of them run
   // at once, two per SM; more CTAs repeat the set-up, fewer leave SMs idle.  Measured for the
@@ -1627,7 +1664,6 @@ int qb_prefix_minima(qb_handle* h, const qb_problem* p, int32_t prefix_bits, dou
   const uint64_t nout = count << sb;
   QB_CUDA(h->exout.ensure(nout * sizeof(qb::ExactOut)));
   const size_t sm = qb::exact_smem_bytes(n, B);
-  QB_CUDA(cudaFuncSetAttribute(qb::exact_records_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
   const uint64_t maxg = 1u << 30;  // sb > 0 only far below it
   for (uint64_t off = 0; off < count; off += maxg) {
     const uint64_t g = std::min<uint64_t>(maxg, count - off);
@@ -1947,7 +1983,6 @@ int noalloc_run(int device, const double* q_dev, int n, int is_integer, int pref
   const qb::ProblemDev pd{n, W};
   noalloc_prep_kernel<<<1, 256, 0, st>>>(q_dev, n, is_integer ? 1 : 0, W, misc);
   const size_t sm0 = qb::gray_gtab_smem(n, a);
-  QB_CUDA(cudaFuncSetAttribute(qb::gray_gtab_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm0));
   qb::gray_gtab_kernel<<<(unsigned)std::min<uint64_t>((1ull << a) / 8 + 1, (uint64_t)sms * 4), 256, sm0, st>>>(pd, a, b, gtab);
   qb::GrayParams gp{};
   gp.P = pd;
@@ -1960,7 +1995,7 @@ int noalloc_run(int device, const double* q_dev, int n, int is_integer, int pref
   gp.gtab = gtab;
   gp.rec = rec;
   const size_t sm1 = qb::gray_pass1_smem(n, a);
-  QB_CUDA(cudaFuncSetAttribute(qb::gray_pass1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm1));
+  QB_CUDA(allow_shared(qb::gray_pass1_kernel));
   qb::gray_pass1_kernel<<<(unsigned)units, qb::kGrayThreads, sm1, st>>>(gp);
   const unsigned rb = (unsigned)std::min<uint64_t>((nrec + 255) / 256, (uint64_t)sms * 8);
   qb::rec_min_kernel<<<rb, 256, 0, st>>>(rec, (int64_t)nrec, &misc->min_key);
@@ -1973,7 +2008,7 @@ int noalloc_run(int device, const double* q_dev, int n, int is_integer, int pref
     maxf = __builtin_popcountll(ff & qb::mask64(n));
   }
   const size_t sm2 = qb::exact_smem_bytes(n, maxf);
-  QB_CUDA(cudaFuncSetAttribute(qb::exact_records_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm2));
+  QB_CUDA(allow_shared(qb::exact_records_kernel));
   qb::exact_records_kernel<<<kNoAllocCands, qb::kExactThreads, sm2, st>>>(pd, rule, geom, cand, &misc->cand_count, 0, 0,
                                                                          eo, 0);
   noalloc_final_kernel<<<1, 256, 0, st>>>(eo, misc, kNoAllocCands, is_integer ? 1 : 0, out_dev);

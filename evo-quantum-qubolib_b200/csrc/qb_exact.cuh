@@ -472,38 +472,42 @@ exact_records_kernel(ProblemDev P, TieRule R, RecGeom G, const uint64_t* __restr
   exact_record_body(P, R, G, rid, out + ((slot << split_bits) | part), smem_d, part, split_bits);
 }
 
-// The candidate records listed in rec_ids[0 .. min(*count_ptr, cap)), each split into
-// 2^split_bits parts, as a grid-stride loop over (record, part) items: the host launches it
-// before it knows the count.  Outputs at (slot << split_bits) | part.
-__global__ void __launch_bounds__(kExactThreads, 2)
-exact_candidates_kernel(ProblemDev P, TieRule R, RecGeom G, const uint64_t* __restrict__ rec_ids,
-                        const int* __restrict__ count_ptr, int cap, int split_bits, ExactOut* __restrict__ out) {
-  extern __shared__ __align__(16) double smem_d[];
-  const int count = min(*count_ptr, cap);
-  const int64_t items = (int64_t)count << split_bits;
-  for (int64_t w = blockIdx.x; w < items; w += gridDim.x) {
-    __syncthreads();  // the previous item's shared-memory readers are done
-    const int64_t slot = w >> split_bits;
-    const int part = (int)(w & ((1 << split_bits) - 1));
-    exact_record_body(P, R, G, rec_ids[slot], out + w, smem_d, part, split_bits);
-  }
-}
+// One solve's control words on the device, uploaded with W and copied back with the answer.
+struct SolveCtl {
+  uint32_t err;      // error word of the tensor-core kernels
+  uint32_t min_key;  // smallest pass-1 record value (f2key)
+  int count;         // candidate records
+  uint32_t done[2];  // CTAs that have finished: exact_candidates_kernel, exact_row_kernel
+  uint32_t pad;
+  ExactOut best;     // exact_candidates_kernel's answer
+  ExactOut row;      // exact_row_kernel's answer
+};
 
-// One CTA: the lexicographic minimum of the first min(*count_ptr, cap) << split_bits
-// outputs into *best (x = 0 with energy 0 and key 0 when *zero_flag is set).
-__global__ void exact_final_kernel(const ExactOut* __restrict__ out, const int* __restrict__ count_ptr, int cap,
-                                   int split_bits, const int* __restrict__ zero_flag, ExactOut* __restrict__ best) {
-  __shared__ double se[32];
-  __shared__ uint64_t sk[32], sx[32];
-  const int64_t items = (int64_t)min(*count_ptr, cap) << split_bits;
+// Every CTA's thread 0 holds b: the last CTA to arrive at *done writes the lexicographic minimum
+// over all of them to *out.  part: gridDim.x entries.
+__device__ __forceinline__ void last_cta_min(const ExactOut& b, ExactOut* __restrict__ part, uint32_t* done,
+                                             ExactOut* __restrict__ out) {
+  __shared__ int last;
+  __shared__ ExactOut red[kExactThreads / 32];
+  if (threadIdx.x == 0) {
+    part[blockIdx.x] = b;
+    __threadfence();
+    last = atomicAdd(done, 1u) == gridDim.x - 1u;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
   double be = __longlong_as_double(0x7ff0000000000000ll);
   uint64_t bk = ~0ull, bx = 0;
-  for (int64_t i = threadIdx.x; i < items; i += blockDim.x)
-    if (lex_less(out[i].e, out[i].key, be, bk)) {
-      be = out[i].e;
-      bk = out[i].key;
-      bx = out[i].x;
+  for (unsigned i = threadIdx.x; i < gridDim.x; i += kExactThreads) {
+    const double e = __ldcg(&part[i].e);
+    const uint64_t k = __ldcg(reinterpret_cast<const unsigned long long*>(&part[i].key));
+    if (lex_less(e, k, be, bk)) {
+      be = e;
+      bk = k;
+      bx = __ldcg(reinterpret_cast<const unsigned long long*>(&part[i].x));
     }
+  }
   for (int off = 16; off; off >>= 1) {
     const double oe = __shfl_down_sync(0xffffffffu, be, off);
     const uint64_t ok = __shfl_down_sync(0xffffffffu, bk, off);
@@ -514,21 +518,58 @@ __global__ void exact_final_kernel(const ExactOut* __restrict__ out, const int* 
       bx = ox;
     }
   }
-  if ((threadIdx.x & 31) == 0) {
-    se[threadIdx.x >> 5] = be;
-    sk[threadIdx.x >> 5] = bk;
-    sx[threadIdx.x >> 5] = bx;
-  }
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ExactOut{be, bk, bx};
   __syncthreads();
   if (threadIdx.x == 0) {
-    for (int w = 1; w < (int)(blockDim.x >> 5); ++w)
-      if (lex_less(se[w], sk[w], be, bk)) {
-        be = se[w];
-        bk = sk[w];
-        bx = sx[w];
+    for (int w = 1; w < kExactThreads / 32; ++w)
+      if (lex_less(red[w].e, red[w].key, be, bk)) {
+        be = red[w].e;
+        bk = red[w].key;
+        bx = red[w].x;
       }
-    *best = *zero_flag ? ExactOut{0.0, 0ull, 0ull} : ExactOut{be, bk, bx};
+    *out = ExactOut{be, bk, bx};
   }
+}
+
+// The candidate records rec_ids[0 .. min(ctl->count, cap)) (rec_ids == nullptr: the records
+// 0 .. count_static), each split into 2^split_bits parts, as a grid-stride loop over (record,
+// part) items: the host launches it before it knows the count.  The lexicographic minimum over
+// all of them goes to ctl->best.
+__global__ void __launch_bounds__(kExactThreads, 2)
+exact_candidates_kernel(ProblemDev P, TieRule R, RecGeom G, const uint64_t* __restrict__ rec_ids, SolveCtl* ctl,
+                        int64_t count_static, int cap, int split_bits, ExactOut* __restrict__ part_out) {
+  extern __shared__ __align__(16) double smem_d[];
+  const int64_t count = rec_ids ? (int64_t)min(ctl->count, cap) : count_static;
+  const int64_t items = count << split_bits;
+  ExactOut b{__longlong_as_double(0x7ff0000000000000ll), ~0ull, 0ull};
+  for (int64_t w = blockIdx.x; w < items; w += gridDim.x) {
+    __syncthreads();  // the previous item's shared-memory readers are done
+    const int64_t slot = w >> split_bits;
+    const int part = (int)(w & ((1 << split_bits) - 1));
+    const ExactOut o = exact_record_min(P, R, G, rec_ids ? rec_ids[slot] : (uint64_t)slot, smem_d, part, split_bits);
+    if (lex_less(o.e, o.key, b.e, b.key)) b = o;
+  }
+  last_cta_min(b, part_out, &ctl->done[0], &ctl->best);
+}
+
+// QB_F1's last step: the smallest 18-bit suffix among the states of ctl->best's prefix with its
+// energy, as the natural-order minimum of that prefix's 2^18 states over gridDim.x = 2^kRowSplit
+// CTAs, into ctl->row (left at +infinity where there is nothing to do).
+constexpr int kRowSplit = 5;
+__global__ void __launch_bounds__(kExactThreads, 2)
+exact_row_kernel(ProblemDev P, SolveCtl* ctl, ExactOut* __restrict__ part_out) {
+  extern __shared__ __align__(16) double smem_d[];
+  ExactOut b{__longlong_as_double(0x7ff0000000000000ll), ~0ull, 0ull};
+  const uint64_t x = ctl->best.x;
+  if (x != 0ull) {
+    RecGeom g{};
+    g.kind = kGeomBlock;
+    g.n = P.n;
+    g.fbits = 18;
+    const TieRule nat{kTieNatural, P.n, 0, 0, 0};
+    b = exact_record_min(P, nat, g, x >> 18, smem_d, (int)blockIdx.x, kRowSplit);
+  }
+  last_cta_min(b, part_out, &ctl->done[1], &ctl->row);
 }
 
 inline size_t exact_smem_bytes(int n, int f) {

@@ -149,6 +149,7 @@ struct TcParams {
   const uint32_t* item_first;  //     [item_first[b], item_first[b + 1])
   int n_max;                // largest n among the items (shared-memory layout)
   unsigned* err;            // error word
+  uint32_t* min_key;        // 16-bit pair kernel, one problem: smallest record value (f2key), or nullptr
   float dmin;               // 16-bit epilogue: lower bound of the accumulator values
   float k0;                 // 16-bit epilogue: 2^23 - dmin, added to the column term
 };
@@ -191,9 +192,6 @@ inline void tc_plan(int n, bool is_int, double abs_sum, int shard_idx, int shard
   p->rec_count = (ge - gb) << 3;
   p->states = (p->tile_end - p->tile_begin) << 15;
 }
-
-// scratch: error word (16 B) + scaled W
-inline size_t tc_scratch_bytes(const TcPlan& p) { return 16 + (size_t)p.n * p.n * sizeof(double); }
 
 #ifdef __CUDACC__
 // ---------------------------------------------------------------- PTX wrappers
@@ -896,25 +894,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_pass1_kernel(TcParams P) {
   }
 }
 
-// scale W into the scratch buffer (float digits keep magnitudes inside the fp16 range)
-__global__ void tc_scale_w_kernel(const double* __restrict__ W, double* __restrict__ out, int nn, double scale) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nn; i += gridDim.x * blockDim.x) out[i] = W[i] * scale;
-}
-
-// clears the error word and writes the scaled W into the scratch buffer
-inline int tc_prepare(const TcPlan& p, ProblemDev pd, void* scratch, cudaStream_t st, int* kernels) {
-  unsigned* err = static_cast<unsigned*>(scratch);
-  double* Wsc = reinterpret_cast<double*>(static_cast<char*>(scratch) + 16);
-  if (cudaMemsetAsync(err, 0, 16, st) != cudaSuccess) return 4;
-  tc_scale_w_kernel<<<8, 256, 0, st>>>(pd.W, Wsc, p.n * p.n, p.scale);
-  ++*kernels;
-  return cudaGetLastError() == cudaSuccess ? 0 : 4;
-}
-
 // the search kernel itself (one persistent CTA per SM)
-inline int tc_launch(const TcPlan& p, float* rec, void* scratch, cudaStream_t st, int sms, int* kernels) {
-  unsigned* err = static_cast<unsigned*>(scratch);
-  double* Wsc = reinterpret_cast<double*>(static_cast<char*>(scratch) + 16);
+// Wsc: W times the plan's scale; err: the error word (cleared)
+inline int tc_launch(const TcPlan& p, float* rec, const double* Wsc, unsigned* err, cudaStream_t st, int sms,
+                     int* kernels) {
   const uint64_t groups = (p.tile_end - p.tile_begin) >> p.gl;
   if (!groups) return 0;
   uint64_t ctas = std::min<uint64_t>((uint64_t)sms, groups);
@@ -940,17 +923,9 @@ inline int tc_launch(const TcPlan& p, float* rec, void* scratch, cudaStream_t st
   // at least 120 KB so that one CTA (and one 512-column TMEM allocation) runs per SM
   const size_t smem = std::max<size_t>(L.total, 120 * 1024) + 1024;
   auto kern = p.u16 ? tc_pass1_kernel<false, true> : tc_pass1_kernel<false, false>;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 4;
   kern<<<(unsigned)ctas, kTcThreads, smem, st>>>(P);
   ++*kernels;
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
-}
-
-inline int tc_check_error(void* scratch, cudaStream_t st) {
-  unsigned e = 0;
-  if (cudaMemcpyAsync(&e, scratch, sizeof(unsigned), cudaMemcpyDeviceToHost, st) != cudaSuccess) return 4;
-  if (cudaStreamSynchronize(st) != cudaSuccess) return 4;
-  return (e & kErrTimeout) ? 5 : 0;
 }
 #endif
 

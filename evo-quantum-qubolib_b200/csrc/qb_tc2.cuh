@@ -1125,6 +1125,7 @@ __global__ void __launch_bounds__(kTc2Threads, 1) tc_pair_kernel(const __grid_co
       const uint4* cpp = reinterpret_cast<const uint4*>(Ct + 8 + hh * 8);
       const int rsh = gl - KW - 1;  // blocks per record: 2^rsh
       float rmin = inf;
+      uint32_t kmin = 0xffffffffu;  // smallest record value of this warp
       const uint32_t full = smem_u32(&acc_full[grp]);
       for (uint32_t p = 0; p < nblk && !fail; ++p) {
         const uint32_t jg = bbase + p, bs = jg & (uint32_t)(kTc2BStages - 1);
@@ -1168,6 +1169,7 @@ __global__ void __launch_bounds__(kTc2Threads, 1) tc_pair_kernel(const __grid_co
         }
         if (((p + 1) >> rsh) != (p >> rsh)) {  // end of a record
           const float wm = warp_min_f(rmin) * inv;
+          if (!kItems) kmin = min(kmin, f2key(wm));
           if (lane == 0) {
             float* dst = rec + (((uint64_t)(p >> rsh) << 3) | ((uint64_t)hh << 2) | (uint64_t)q);
             if (wm >= 0.f)
@@ -1178,6 +1180,7 @@ __global__ void __launch_bounds__(kTc2Threads, 1) tc_pair_kernel(const __grid_co
           rmin = inf;
         }
       }
+      if (!kItems && lane == 0 && P.min_key) atomicMin(P.min_key, kmin);
       ok = !fail;
     }
     if (!ok) {
@@ -1200,10 +1203,10 @@ __global__ void __launch_bounds__(kTc2Threads, 1) tc_pair_kernel(const __grid_co
 
 // the pair-form search kernel (one persistent CTA per SM); gamma = couplings of variable
 // n-16 with u bits 0..7, in the units of the scaled W
-inline int tc2_launch(const TcPlan& p, const float* gamma, float* rec, void* scratch, cudaStream_t st, int sms,
-                      int* kernels) {
-  unsigned* err = static_cast<unsigned*>(scratch);
-  double* Wsc = reinterpret_cast<double*>(static_cast<char*>(scratch) + 16);
+// Wsc: W times the plan's scale; err: the error word (cleared); min_key: receives the smallest
+// record value (16-bit form; initially 0xffffffff)
+inline int tc2_launch(const TcPlan& p, const float* gamma, float* rec, const double* Wsc, unsigned* err,
+                      uint32_t* min_key, cudaStream_t st, int sms, int* kernels) {
   const uint64_t groups = (p.tile_end - p.tile_begin) >> p.gl;
   if (!groups) return 0;
   uint64_t ctas = std::min<uint64_t>((uint64_t)sms, groups);
@@ -1223,6 +1226,7 @@ inline int tc2_launch(const TcPlan& p, const float* gamma, float* rec, void* scr
   P.groups_per_cta = gpc;
   P.rec = rec;
   P.err = err;
+  P.min_key = min_key;
   P.stall = p.stall ? 1 : 0;
   for (int k = 0; k < 32; ++k) {
     float g = 0.f;
@@ -1240,7 +1244,6 @@ inline int tc2_launch(const TcPlan& p, const float* gamma, float* rec, void* scr
   const TcSmemLayout L = tc_layout(p.n);
   const size_t smem = p.u16 ? tc2_smem_bytes(p.n) : std::max<size_t>(L.total + kTcBStages * 128 * 4, 120 * 1024) + 1024;
   auto* kern = p.u16 ? tc_pair_kernel<false> : tc_pair_fp32_kernel;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 4;
   kern<<<(unsigned)ctas, p.u16 ? kTc2Threads : kTcThreads, smem, st>>>(Q);
   ++*kernels;
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
