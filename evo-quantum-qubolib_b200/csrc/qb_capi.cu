@@ -1657,7 +1657,7 @@ int qb_prefix_minima(qb_handle* h, const qb_problem* p, int32_t prefix_bits, dou
   const uint64_t count = 1ull << A;
   // few prefixes: each split over 2^sb CTAs (of at least 2^14 states) as long as all of them run
   // at once, two per SM; more CTAs repeat the set-up, fewer leave SMs idle.  Measured for the
-  // whole call (us) at sb = 0 1 2 3 4 5: n = 27, A = 7 182 128 132 149 167 221; n = 24, A = 4
+  // whole call (us, the winner's thread walking again) at sb = 0 1 2 3 4 5: n = 27, A = 7 182 128 132 149 167 221; n = 24, A = 4
   // 177 113 77 56 52 58; n = 23, A = 3 176 112 77 55 52 43; n = 30, A = 10 683 672 738 864
   int sb = 0;
   while (sb < B - 14 && (count << (sb + 1)) <= 2ull * (uint64_t)h->sm_count) ++sb;

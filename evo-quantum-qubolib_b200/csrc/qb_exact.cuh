@@ -9,9 +9,10 @@
 // depend on the thread and on h, and their own couplings).  A walk step that flips variable o
 // costs one add and one minimum per state: el[g] += +- sum of W_og over the set bits (a table in
 // shared memory, the same for every thread), one c update, and the update of the walked
-// variables' fields.  Only the minimum is kept on the way; the threads within rounding of the
-// CTA's minimum (usually one) walk again to find the state, with the tie key, and the winner's
-// energy is summed from scratch, so the reported value does not carry the walk's rounding.
+// variables' fields.  Only the minimum and its step are kept on the way; the threads within rounding of
+// the CTA's minimum (usually one) then look for the state at that step (walking again where several
+// steps attain the minimum), with the tie key, and the winner's energy is summed from scratch, so
+// the reported value does not carry the walk's rounding.
 //
 // What bounds it: for one candidate record of 2^17 states in 16 parts (a 36-variable solve) the
 // latency of one CTA's steps -- W from L2, the base state's fields and the start tables (all
@@ -19,7 +20,8 @@
 // when every thread summed its start and its best state's energy alone (n = 20 .. 37; 2^19-state
 // records of n = 40 158 -> 33 us).  Many states per CTA (2^19, qb_prefix_minima at n = 27): per
 // state one FP64 add and one FP64 compare with two selects, two CTAs per SM (128 registers);
-// 2^27 states 520 -> 105 us.  The 4096-problem batch's pass 2 1400 -> 730 us.
+// 2^27 states 520 -> 69 us (105 when the winner's thread always walked again: seven of a CTA's
+// eight warps waited for it).  The 4096-problem batch's pass 2 1400 -> 507 us.
 #pragma once
 #include <cstring>
 
@@ -347,10 +349,12 @@ __device__ __forceinline__ ExactOut exact_record_min(const ProblemDev& P, const 
     }
   };
   const uint32_t steps = 1u << Lo;
-  // pass 0: the minimum.  Pass 1, the threads that can hold the winner: the smallest key among
-  // the thread's states of minimal energy.
+  // pass 0: the minimum, the walk step that first attains it and how many do.  Pass 1, the
+  // threads that can hold the winner: the smallest key among the thread's states of minimal
+  // energy, at that step (its el summed from the start) or, with several, by walking again.
   double best_e = inf, m = inf;
   uint64_t best_k = ~0ull, best_x = 0;
+  uint32_t best_st = 0, best_cnt = 0;
   bool cand = active;
   // exact sums: the threads at the CTA's minimum; otherwise those within twice the walk's
   // rounding of it (per step and for the start's about 100 additions, 2^-53 sum |W| each)
@@ -361,15 +365,40 @@ __device__ __forceinline__ ExactOut exact_record_min(const ProblemDev& P, const 
     if (cand) {
       if (pass == 0 || steps > 1) start();  // without walked bits el still holds the start
       uint64_t Xh = 0;
+      uint32_t st = 0;
+      double target = best_e;
+      const bool seek = pass == 1 && best_cnt == 1;
+      if (seek) {
+        st = best_st;
+        uint32_t h = st ^ (st >> 1), lower = 0;
 #pragma unroll 1
-      for (uint32_t st = 0;;) {
+        for (; h; h &= h - 1) {
+          const int o = __ffs(h) - 1;
+          const double* row = Ws + var[Lr + o] * n;
+          double d = row[var[Lr + o]] + at[o * kExactThreads + t];
+          for (uint32_t l = lower; l; l &= l - 1) d += row[var[Lr + __ffs(l) - 1]];
+          c += d;
+          lower |= 1u << o;
+          Xh |= 1ull << (n - 1 - var[Lr + o]);
+#pragma unroll
+          for (int g = 0; g < 32; ++g) el[g] += T[o * 32 + g];
+        }
+        target = c + min32d(el);
+      }
+#pragma unroll 1
+      for (;;) {
         const double e = c + min32d(el);
         if (pass == 0) {
-          best_e = e < best_e ? e : best_e;
-        } else if (e == best_e) {
+          if (e < best_e) {
+            best_e = e;
+            best_st = st;
+            best_cnt = 0;
+          }
+          best_cnt += e == best_e;
+        } else if (e == target) {
           uint32_t hit = 0;
 #pragma unroll
-          for (int g = 0; g < 32; ++g) hit |= c + el[g] == best_e ? 1u << g : 0u;
+          for (int g = 0; g < 32; ++g) hit |= c + el[g] == target ? 1u << g : 0u;
           uint64_t Xt = base | Xh;
           for (int j = 0; j < tb; ++j)
             if ((t >> j) & 1) Xt |= 1ull << (n - 1 - var[L + j]);
@@ -386,7 +415,7 @@ __device__ __forceinline__ ExactOut exact_record_min(const ProblemDev& P, const 
             }
           }
         }
-        if (++st == steps) break;
+        if (seek || ++st == steps) break;
         step(st);
         Xh ^= 1ull << (n - 1 - var[Lr + __ffs(st) - 1]);
       }

@@ -300,9 +300,11 @@ __device__ __forceinline__ void tc_issue_n128(uint32_t dtmem, uint64_t adesc, ui
 }
 
 // bounded wait of a role with slack (the tile walk and the B producer, up to 64 blocks and 4
-// B stages ahead): sleeps between polls so that it leaves the issue slots to the epilogue
+// B stages ahead): sleeps between polls so that it leaves the issue slots to the epilogue,
+// after a few polls without sleep (the pipeline's start, where nothing is ahead yet)
 __device__ __forceinline__ bool mbar_wait_idle(uint64_t* b, uint32_t parity, volatile int* abort_flag) {
-  if (mbar_try_wait(b, parity)) return true;
+  for (int it = 0; it < 16; ++it)
+    if (mbar_try_wait(b, parity)) return true;
   const uint64_t t0 = globaltimer_ns();
   for (;;) {
     __nanosleep(1000);
@@ -790,20 +792,26 @@ __global__ void __launch_bounds__(kTc2Threads, 1) tc_pair_kernel(const __grid_co
                  P.inv_scale};
   }
 
-  if (tid == 0) {
-    for (int s = 0; s < kTcParamSlots; ++s) {
-      mbar_init(&p_full[s], 1);
-      mbar_init(&p_empty[s], 1);
+  // the item's W into shared memory, its records to +infinity, its corrections
+  auto load_item = [&](uint32_t it) {
+    const TcItem I = kItems ? P.items[it] : one;
+    const Tc2Tab& Tb = kItems ? Q.tabs[it] : Q.tab;
+    for (int i = tid; i < I.n * I.n; i += kTc2Threads) Ws[i] = I.W[i];
+    for (uint64_t r = (uint64_t)tid; r < ((I.ntiles >> I.gl) << 3); r += kTc2Threads) I.rec[r] = __int_as_float(0x7f800000);
+    if (tid < 24) Ct[tid] = tid < 8 ? Tb.corr_t[0][tid] : Tb.corr_p[0][(tid - 8) >> 3][tid & 7];
+  };
+  if (tid < kTcParamSlots) {
+    mbar_init(&p_full[tid], 1);
+    mbar_init(&p_empty[tid], 1);
+    if (tid < kTc2BStages) {
+      mbar_init(&b_full[tid], 1);
+      mbar_init(&b_empty[tid], 4 * kTc2Groups);  // every epilogue warp
     }
-    for (int s = 0; s < kTc2BStages; ++s) {
-      mbar_init(&b_full[s], 1);
-      mbar_init(&b_empty[s], 4 * kTc2Groups);  // every epilogue warp
+    if (tid < kTc2Groups) {
+      mbar_init(&acc_full[tid], 1);
+      mbar_init(&acc_empty[tid], 4);
     }
-    for (int s = 0; s < kTc2Groups; ++s) {
-      mbar_init(&acc_full[s], 1);
-      mbar_init(&acc_empty[s], 4);
-    }
-    *abort_flag = 0;
+    if (tid == 0) *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -813,16 +821,27 @@ __global__ void __launch_bounds__(kTc2Threads, 1) tc_pair_kernel(const __grid_co
   // A operands (constant, the same for every item), one per low pattern st: A[y][i] = y_i
   // (i < 7); the column term's digits (slots 8-10) 1, 2048, 32768; low t bit m (slots
   // kLowSlot[m], kLowSlot[m] + 1, or 7 and 15) bit m of st times 1, 2048
-  for (int e = tid; e < NS * 128 * 16; e += kTc2Threads) {
-    const int st = e >> 11, y = (e >> 4) & 127, k = e & 15;
-    float v;
-    if (k < 7)
-      v = (float)((y >> k) & 1);
-    else if (k >= 8 && k < 11)
-      v = k == 8 ? 1.0f : (k == 9 ? 2048.0f : 32768.0f);
-    else
-      v = ((st >> tc2_low_bit(k)) & 1) ? (tc2_low_digit(k) ? 2048.0f : 1.0f) : 0.0f;
-    *reinterpret_cast<__half*>(Asm + st * 128 * 32 + kmaj_off(y, k)) = __float2half_rn(v);
+  load_item(it_lo);
+  for (int e = tid; e < NS * 128 * 2; e += kTc2Threads) {  // 8 columns (16 bytes) at a time
+    const int st = e >> 8, y = (e >> 1) & 127, kh = e & 1;
+    constexpr uint32_t h1 = 0x3C00u, h2048 = 0x6800u, h32768 = 0x7800u;  // f16 1, 2048, 32768
+    uint32_t w[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      uint32_t h[2];
+#pragma unroll
+      for (int d = 0; d < 2; ++d) {
+        const int kl = 2 * c + d, kg = 8 + kl;  // column kl, or kg in the upper half
+        const uint32_t lo = kl < 7 ? (((y >> kl) & 1) ? h1 : 0u) : (((st >> tc2_low_bit(7)) & 1) ? h2048 : 0u);
+        const uint32_t hi = kg == 8 ? h1
+                            : kg == 9 ? h2048
+                            : kg == 10 ? h32768
+                                       : (((st >> tc2_low_bit(kg)) & 1) ? (tc2_low_digit(kg) ? h2048 : h1) : 0u);
+        h[d] = kh ? hi : lo;
+      }
+      w[c] = h[0] | (h[1] << 16);
+    }
+    *reinterpret_cast<uint4*>(Asm + st * 128 * 32 + kmaj_off(y, kh * 8)) = make_uint4(w[0], w[1], w[2], w[3]);
   }
   tc_fence_before();
   __syncthreads();
@@ -840,101 +859,116 @@ __global__ void __launch_bounds__(kTc2Threads, 1) tc_pair_kernel(const __grid_co
     const uint32_t bbase = kItems ? bnext : 0u;
 
     // ------------------------------------------------------------ per-item set-up
-    for (int i = tid; i < n * n; i += kTc2Threads) Ws[i] = I.W[i];
-    for (uint64_t r = (uint64_t)tid; r < ((I.ntiles >> gl) << 3); r += kTc2Threads) rec[r] = __int_as_float(0x7f800000);
-    if (tid < 24) Ct[tid] = tid < 8 ? Tb.corr_t[0][tid] : Tb.corr_p[0][(tid - 8) >> 3][tid & 7];
-    __syncthreads();
+    // Tables from W, FP64, without branches on the patterns' bits; different warps build
+    // different ones.  (n = 20: the whole kernel 31 -> 18 thousand cycles.)
+    const int kb0 = n - 17 - KW;  // variable of block bit 0 (block bit k: kb0 - k)
+    if (warp < 8) {
+      // the column term's constant part E_U(u) + X(u) + 2^23 - Dlow, u = tid
+      const int u = tid;
+      double e = 0.0;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const double* row = Ws + (n - 1 - j) * n;
+        double r = row[n - 1 - j];
+#pragma unroll
+        for (int j2 = 0; j2 < j; ++j2) r += ((u >> j2) & 1) ? row[n - 1 - j2] : 0.0;
+        e += ((u >> j) & 1) ? r : 0.0;
+      }
+      const double x = ((u >> 4) & 1 ? (double)Tb.gx[0] : 0.0) + ((u >> 5) & 1 ? (double)Tb.gx[1] : 0.0) +
+                       ((u >> 6) & 1 ? (double)Tb.gx[2] : 0.0);
+      EU[u] = (float)(rint(e) + x + (double)Tb.k0s[0]);
+    } else if (warp < 12) {
+      // low t bits (pattern p = 2 st + b: bit 0 the pair's) x row couplings, y = tid - 256
+      const int y = tid - 256;
+      double r[KW + 1], v[2 * NS];
+#pragma unroll
+      for (int m = 0; m <= KW; ++m) {
+        const double* row = Ws + (n - 16 - m) * n;
+        r[m] = 0.0;
+#pragma unroll
+        for (int i = 0; i < 7; ++i) r[m] += ((y >> i) & 1) ? row[n - 9 - i] : 0.0;
+      }
+      v[0] = 0.0;
+#pragma unroll
+      for (int m = 0; m <= KW; ++m)
+#pragma unroll
+        for (int p = 0; p < (1 << m); ++p) v[(1 << m) + p] = v[p] + r[m];
+#pragma unroll
+      for (int st = 0; st < NS; ++st) WL[st * 128 + y] = make_float2((float)v[2 * st], (float)v[2 * st + 1]);
+    } else if (warp < 16) {
+      const int y = tid - 384;
+      double e = 0.0;
+#pragma unroll
+      for (int i = 0; i < 7; ++i) {
+        const double* row = Ws + (n - 9 - i) * n;
+        double r = row[n - 9 - i];
+#pragma unroll
+        for (int i2 = 0; i2 < i; ++i2) r += ((y >> i2) & 1) ? row[n - 9 - i2] : 0.0;
+        e += ((y >> i) & 1) ? r : 0.0;
+      }
+      EY[y] = (float)e;
+      if (y < 2 * NS) {  // energy of the low t bits' pattern y alone
+        double v = 0.0;
+#pragma unroll
+        for (int m = 0; m <= KW; ++m) {
+          const double* row = Ws + (n - 16 - m) * n;
+          double r = row[n - 16 - m];
+#pragma unroll
+          for (int m2 = 0; m2 < m; ++m2) r += ((y >> m2) & 1) ? row[n - 16 - m2] : 0.0;
+          v += ((y >> m) & 1) ? r : 0.0;
+        }
+        LL[y] = (float)v;
+      }
+    } else {
+      // LO[p]: the five lowest block bits' pattern p: couplings with u (8), y (7), the low t
+      // bits (KW + 1) and their own energy (block bits beyond the problem's are never set)
+      for (int e = tid - 512; e < 32 * kTc2LoCols; e += 128) {
+        const int p = e & 31, c = e >> 5;
+        double v = 0.0;
+        if (c == kTc2LoCols - 1) {
+#pragma unroll
+          for (int b = 0; b < 5; ++b) {
+            if (b > kb0) break;
+            const double* row = Ws + (kb0 - b) * n;
+            double r = row[kb0 - b];
+#pragma unroll
+            for (int b2 = 0; b2 < b; ++b2) r += ((p >> b2) & 1) ? row[kb0 - b2] : 0.0;
+            v += ((p >> b) & 1) ? r : 0.0;
+          }
+        } else {
+          const int col = c < 8 ? n - 1 - c : c < 15 ? n - 9 - (c - 8) : n - 16 - (c - 15);
+#pragma unroll
+          for (int b = 0; b < 5; ++b) {
+            if (b > kb0) break;
+            v += ((p >> b) & 1) ? Ws[(kb0 - b) * n + col] : 0.0;
+          }
+        }
+        LO[p * kTc2LoCols + c] = v;
+      }
+    }
     // B operand, constant columns: coupling rows of the y variables (one exact fp16 integer
     // each) and of the low t bits (two exact digits each)
     for (int e = tid; e < kTcN * 10; e += kTc2Threads) {
       const int u = e & (kTcN - 1), i = e >> 8;  // i < 7: y variable i; else low t bit i - 7
       const double* row = Ws + (i < 7 ? n - 9 - i : n - 17 - (i - 7)) * n;
       double v = 0.0;
-      for (int j = 0; j < 8; ++j)
-        if ((u >> j) & 1) v += row[n - 1 - j];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v += ((u >> j) & 1) ? row[n - 1 - j] : 0.0;
       const float r = (float)rint(v);
       if (i < 7) {
         const __half hv = __float2half_rn(r);
+#pragma unroll
         for (int s = 0; s < kTc2BStages; ++s) *reinterpret_cast<__half*>(Bsm + s * kTcN * 32 + kmaj_off(u, i)) = hv;
       } else {
         const float d1 = floorf(r * (1.0f / 2048.0f));
         const __half h0 = __float2half_rn(fmaf(-2048.0f, d1, r)), h1 = __float2half_rn(d1);
         const int k0 = tc2_low_slot(i - 7, 0), k1 = tc2_low_slot(i - 7, 1);
+#pragma unroll
         for (int s = 0; s < kTc2BStages; ++s) {
           *reinterpret_cast<__half*>(Bsm + s * kTcN * 32 + kmaj_off(u, k0)) = h0;
           *reinterpret_cast<__half*>(Bsm + s * kTcN * 32 + kmaj_off(u, k1)) = h1;
         }
       }
-    }
-    // the column term's constant part E_U(u) + X(u) + 2^23 - Dlow
-    for (int u = tid; u < kTcN; u += kTc2Threads) {
-      double e = 0.0;
-      for (int j = 0; j < 8; ++j) {
-        if (!((u >> j) & 1)) continue;
-        const double* row = Ws + (n - 1 - j) * n;
-        e += row[n - 1 - j];
-        for (int j2 = 0; j2 < j; ++j2)
-          if ((u >> j2) & 1) e += row[n - 1 - j2];
-      }
-      const double x = ((u >> 4) & 1 ? (double)Tb.gx[0] : 0.0) + ((u >> 5) & 1 ? (double)Tb.gx[1] : 0.0) +
-                       ((u >> 6) & 1 ? (double)Tb.gx[2] : 0.0);
-      EU[u] = (float)(rint(e) + x + (double)Tb.k0s[0]);
-    }
-    for (int y = tid; y < 128; y += kTc2Threads) {
-      double e = 0.0;
-      for (int i = 0; i < 7; ++i) {
-        if (!((y >> i) & 1)) continue;
-        const double* row = Ws + (n - 9 - i) * n;
-        e += row[n - 9 - i];
-        for (int i2 = 0; i2 < i; ++i2)
-          if ((y >> i2) & 1) e += row[n - 9 - i2];
-      }
-      EY[y] = (float)e;
-    }
-    // low t bits (pattern p = 2 st + b: bit 0 the pair's) x row couplings, and their own energies
-    for (int e = tid; e < NS * 128 * 2; e += kTc2Threads) {
-      const int b = e & 1, y = (e >> 1) & 127, st = e >> 8;
-      const int p = 2 * st + b;
-      double v = 0.0;
-      for (int m = 0; m <= KW; ++m) {
-        if (!((p >> m) & 1)) continue;
-        const double* row = Ws + (n - 16 - m) * n;
-        for (int i = 0; i < 7; ++i)
-          if ((y >> i) & 1) v += row[n - 9 - i];
-      }
-      reinterpret_cast<float*>(WL)[e] = (float)v;
-    }
-    for (int p = tid; p < 2 * NS; p += kTc2Threads) {
-      double v = 0.0;
-      for (int m = 0; m <= KW; ++m) {
-        if (!((p >> m) & 1)) continue;
-        const double* row = Ws + (n - 16 - m) * n;
-        v += row[n - 16 - m];
-        for (int m2 = 0; m2 < m; ++m2)
-          if ((p >> m2) & 1) v += row[n - 16 - m2];
-      }
-      LL[p] = (float)v;
-    }
-    // LO[p]: the five lowest block bits' pattern p: couplings with u (8), y (7), the low t
-    // bits (KW + 1) and their own energy
-    const int kb0 = n - 17 - KW;  // variable of block bit 0 (block bit k: kb0 - k)
-    for (int e = tid; e < 32 * kTc2LoCols; e += kTc2Threads) {
-      const int p = e / kTc2LoCols, c = e % kTc2LoCols;
-      double v = 0.0;
-      if (c == kTc2LoCols - 1) {
-        for (int k = 0; k < 5; ++k) {
-          if (!((p >> k) & 1) || k > kb0) continue;
-          const double* row = Ws + (kb0 - k) * n;
-          v += row[kb0 - k];
-          for (int k2 = 0; k2 < k; ++k2)
-            if ((p >> k2) & 1) v += row[kb0 - k2];
-        }
-      } else {
-        const int col = c < 8 ? n - 1 - c : c < 15 ? n - 9 - (c - 8) : n - 16 - (c - 15);
-        for (int k = 0; k < 5; ++k)
-          if (((p >> k) & 1) && k <= kb0) v += Ws[(kb0 - k) * n + col];
-      }
-      LO[e] = v;
     }
     fence_proxy_async();
     tc_fence_before();
@@ -1192,6 +1226,10 @@ __global__ void __launch_bounds__(kTc2Threads, 1) tc_pair_kernel(const __grid_co
     tc_fence_after();
     bnext = bbase + nblk;
     if (*abort_flag) break;  // uniform: read after the barrier
+    if (kItems && it + 1 < it_hi) {
+      load_item(it + 1);
+      __syncthreads();
+    }
   }
   tc_fence_before();
   __syncthreads();
