@@ -8,7 +8,8 @@
 //                           CTA runs a list of (problem, run of record blocks) items
 //   3. batch_select_kernel  per problem: smallest record, threshold, candidate records
 //   4. batch_exact_kernel   exact FP64 re-evaluation of every candidate record -- and, for
-//                           problems with n < 20, of all their records (the whole search)
+//                           problems with n < 20, of all their records (the whole search);
+//                           as many CTAs as run at once take the records in turn
 //   5. batch_key_kernel     per problem: smallest order key among the states of minimal E
 // Per-problem minima are combined with 64-bit atomics on an order-preserving encoding of
 // the FP64 energy, then on the tie-rule key, which maps one-to-one to the state.
@@ -150,19 +151,28 @@ __global__ void batch_select_kernel(const BatchInst* __restrict__ insts, const u
   }
 }
 
-// 4. exact evaluation of candidate s = blockIdx.x (s < min(count, cap))
+// 4. exact evaluation of the candidates s < min(count, cap), taken in turn by the CTAs (*next
+// starts at 0)
 __global__ void __launch_bounds__(kExactThreads, 2)
 batch_exact_kernel(const BatchInst* __restrict__ insts, const double* __restrict__ W,
                    const BatchCand* __restrict__ cand, const int* __restrict__ cand_count, int cap,
-                   ExactOut* __restrict__ out, uint64_t* __restrict__ emin) {
+                   unsigned* __restrict__ next, ExactOut* __restrict__ out, uint64_t* __restrict__ emin) {
   extern __shared__ __align__(16) double bex_smem[];
-  const int count = min(*cand_count, cap);
-  if ((int)blockIdx.x >= count) return;
-  const BatchCand c = cand[blockIdx.x];
-  const BatchInst I = insts[c.inst];
-  exact_record_body(batch_problem(I, W), batch_rule(I), batch_geom(I), c.rid, out + blockIdx.x, bex_smem);
-  if (threadIdx.x == 0) atomicMin(reinterpret_cast<unsigned long long*>(emin + c.inst),
-                                  (unsigned long long)ord_f64(out[blockIdx.x].e));
+  __shared__ unsigned slot;
+  const unsigned count = (unsigned)min(*cand_count, cap);
+  for (;;) {
+    if (threadIdx.x == 0) slot = atomicAdd(next, 1u);
+    __syncthreads();  // also: the previous candidate's shared-memory readers are done
+    const unsigned s = slot;
+    if (s >= count) return;
+    const BatchCand c = cand[s];
+    const BatchInst I = insts[c.inst];
+    const ExactOut o = exact_record_min(batch_problem(I, W), batch_rule(I), batch_geom(I), c.rid, bex_smem, 0, 0);
+    if (threadIdx.x == 0) {
+      out[s] = o;
+      atomicMin(reinterpret_cast<unsigned long long*>(emin + c.inst), (unsigned long long)ord_f64(o.e));
+    }
+  }
 }
 
 // 5. smallest key among each problem's minimal-energy candidates

@@ -38,7 +38,7 @@ struct DevBuf {
     if (p) cudaFree(p);
     p = nullptr;
     cap = 0;
-    size_t want = std::max<size_t>(bytes, 256);
+    const size_t want = std::max<size_t>(bytes + bytes / 8, 256);  // room for the next batch, a little larger
     cudaError_t e = cudaMalloc(&p, want);
     if (e == cudaSuccess) cap = want;
     return e;
@@ -58,7 +58,7 @@ struct HostBuf {
     if (p) cudaFreeHost(p);
     p = nullptr;
     cap = 0;
-    size_t want = std::max<size_t>(bytes, 4096);
+    const size_t want = std::max<size_t>(bytes + bytes / 8, 4096);
     cudaError_t e = cudaMallocHost(&p, want);
     if (e == cudaSuccess) cap = want;
     return e;
@@ -119,10 +119,10 @@ struct qb_handle_s {
   int device = 0;
   cudaStream_t own = nullptr;
   cudaStream_t st = nullptr;
-  DevBuf W;  // SolveCtl, W (n*n doubles), W times the tensor-core plan's scale (n*n doubles)
+  DevBuf W;  // SolveCtl, then W (n*n doubles)
   DevBuf gtab, rec, cand, misc, exout;
-  DevBuf bat[15];  // qb_solve_batch: W, insts, gtab items, unit items, selection ids, cands, out, G tables,
-                   // records, minima, scaled W, tensor-core items, item ranges, error word
+  DevBuf bat[15];  // qb_solve_batch: 0 W, 1 the small arrays and candidates, 6 outputs, 7 G tables, 8 records;
+                   // QB_F1's int16 form: 0 Q, 6 BB, 7 ABBA, 8 AA, 9 keys and answer
   HostBuf hW, hmisc, hout, hbat;  // hW: the upload of W; hbat: qb_solve_batch's packed W matrices (pinned)
   HostBuf hraw;                    // a device matrix copied back (pinned)
   HostBuf hstage;                  // qb_solve_batch: descriptors and work lists (pinned)
@@ -371,20 +371,15 @@ static_assert(sizeof(qb::SolveCtl) <= kCtlBytes, "control block");
 qb::SolveCtl* dev_ctl(qb_handle* h) { return static_cast<qb::SolveCtl*>(h->W.p); }
 const double* dev_W(qb_handle* h) { return reinterpret_cast<const double*>(static_cast<char*>(h->W.p) + kCtlBytes); }
 
-// One copy: the control block at its initial values, W and, with scale != 0, W times scale
-// behind it.
-int upload_W(qb_handle* h, const std::vector<double>& W, double scale = 0.0) {
-  const size_t nn = W.size();
-  const size_t bytes = kCtlBytes + (scale != 0.0 ? 2 : 1) * nn * sizeof(double);
+// One copy: the control block at its initial values, and W.
+int upload_W(qb_handle* h, const std::vector<double>& W) {
+  const size_t bytes = kCtlBytes + W.size() * sizeof(double);
   QB_CUDA(h->hW.ensure(bytes));
-  QB_CUDA(h->W.ensure(kCtlBytes + 2 * nn * sizeof(double)));
+  QB_CUDA(h->W.ensure(bytes));
   qb::SolveCtl c{};
   c.min_key = 0xffffffffu;
   memcpy(h->hW.p, &c, sizeof(c));
-  double* dst = reinterpret_cast<double*>(static_cast<char*>(h->hW.p) + kCtlBytes);
-  memcpy(dst, W.data(), nn * sizeof(double));
-  if (scale != 0.0)
-    for (size_t i = 0; i < nn; ++i) dst[nn + i] = W[i] * scale;
+  memcpy(static_cast<char*>(h->hW.p) + kCtlBytes, W.data(), W.size() * sizeof(double));
   QB_CUDA(cudaMemcpyAsync(h->W.p, h->hW.p, bytes, cudaMemcpyHostToDevice, h->st));
   h->h2d += (int64_t)bytes;
   return QB_OK;
@@ -440,10 +435,9 @@ int run_pass1(qb_handle* h, Plan& P) {
   }
   h->main0 = 0;  // nothing before the search kernel
   unsigned* err = &dev_ctl(h)->err;
-  const double* Wsc = dev_W(h) + (size_t)P.n * P.n;
-  const int rc = P.tc.pair ? qb::tc2_launch(P.tc, P.tc.gamma, static_cast<float*>(h->rec.p), Wsc, err,
+  const int rc = P.tc.pair ? qb::tc2_launch(P.tc, P.tc.gamma, static_cast<float*>(h->rec.p), pd.W, err,
                                             &dev_ctl(h)->min_key, h->st, h->sm_count, &h->kernels)
-                           : qb::tc_launch(P.tc, static_cast<float*>(h->rec.p), Wsc, err, h->st, h->sm_count, &h->kernels);
+                           : qb::tc_launch(P.tc, static_cast<float*>(h->rec.p), pd.W, err, h->st, h->sm_count, &h->kernels);
   if (rc) return rc;
   QB_CUDA(cudaEventRecord(h->ev[5], h->st));
   return QB_OK;
@@ -602,7 +596,7 @@ int begin_launch(qb_handle* h, const qb_problem* p, const qb_options* o, Plan& P
                  (P.tc.pair ? qb::tc2_u16_eligible(P.n, W.data(), &P.tc.dmin) : qb::tc_u16_eligible(P.n, W.data(), &P.tc.dmin));
     }
   }
-  rc = upload_W(h, W, P.form == QB_FORM_TC ? P.tc.scale : 0.0);
+  rc = upload_W(h, W);
   if (rc) return rc;
   QB_CUDA(h->misc.ensure(64));
   QB_CUDA(h->hmisc.ensure(64));
@@ -659,9 +653,9 @@ int begin_finish_pass1(qb_handle* h, Plan& P, double* local_min) {
 // qb_solve of one whole problem: after pass 1 the minimum, the selection, the exact
 // re-evaluation and the final pick (with QB_F1's suffix step) follow on the device, then one copy
 // of the control block to the host.  The 16-bit pair kernel reduces its records' minimum itself,
-// so that a solve is three launches (four under QB_F1's rule): 65 us of device time against 107
-// at n = 20 .. 28 with the scaling, threshold and final kernels and the clears on their own, and
-// one host round trip against five under QB_F1's rule.  Returns -1 when the candidates overflow
+// so that a solve is three launches (four under QB_F1's rule) and one round trip; the whole call
+// at n = 20 .. 28 took 107 us with the scaling, threshold and final kernels and the clears on
+// their own (84 us without them), and 165 us with QB_F1's five round trips (94 us).  Returns -1 when the candidates overflow
 // the cap (the caller then takes the two-phase path with a larger cap).
 int solve_fused(qb_handle* h, const Plan& P, qb_result* r) {
   qb::SolveCtl* ctl = dev_ctl(h);
@@ -1080,12 +1074,12 @@ constexpr int kBatchMaxN = 36;            // larger problems are solved one by o
 constexpr int kBatchTcMinN = 24;          // from here on the tensor-core form (>= 512 tiles)
 constexpr uint64_t kBatchGtabChunk = 1024;  // G-table steps per CTA
 
-// fn(lo, hi) over [0, count) split into contiguous ranges on up to 16 threads (one thread for
-// small counts)
+// fn(lo, hi) over [0, count) split into contiguous ranges on up to 16 threads, one per 32768
+// units of work (a thread costs about 25 us to start and join: 20 us of converting matrices)
 template <class F>
-void parallel_ranges(int count, F fn) {
+void parallel_ranges(int count, uint64_t work, F fn) {
   const int hw = (int)std::max(1u, std::thread::hardware_concurrency());
-  const int nt = std::max(1, std::min({16, hw, count / 64}));
+  const int nt = (int)std::max<uint64_t>(1, std::min<uint64_t>({16, (uint64_t)hw, (uint64_t)count, work / 32768}));
   if (nt <= 1) {
     fn(0, count);
     return;
@@ -1098,29 +1092,29 @@ void parallel_ranges(int count, F fn) {
   for (auto& x : th) x.join();
 }
 
-// Host -> device copies of qb_solve_batch's small arrays, staged in one pinned buffer so that
-// every copy reads from a stable address (a captured graph replays the same copies)
-struct Stage {
-  struct Copy {
-    void* dst;
+// qb_solve_batch's small arrays: laid out in one device buffer and mirrored in one pinned host
+// buffer, so that one copy from a stable address carries them all (a captured graph replays it)
+struct Arena {
+  struct Part {
+    const void* src;
     size_t off, bytes;
   };
-  std::vector<unsigned char> bytes;  // assembled here, then copied into the pinned buffer once
-  std::vector<Copy> copies;
+  size_t size = 0;
+  std::vector<Part> parts;
   template <class T>
-  void add(void* dst, const std::vector<T>& v) {
-    const size_t off = (bytes.size() + 15) & ~(size_t)15;
-    bytes.resize(off + v.size() * sizeof(T));
-    if (!v.empty()) memcpy(bytes.data() + off, v.data(), v.size() * sizeof(T));
-    if (!v.empty()) copies.push_back(Copy{dst, off, v.size() * sizeof(T)});
+  size_t add(const std::vector<T>& v) {  // v must not move or change until fill()
+    return add_raw(v.data(), v.size() * sizeof(T));
+  }
+  size_t add_raw(const void* src, size_t bytes) {  // src == nullptr: room filled by the caller
+    const size_t off = (size + 15) & ~(size_t)15;
+    if (src && bytes) parts.push_back(Part{src, off, bytes});
+    size = off + bytes;
+    return off;
+  }
+  void fill(void* host) const {
+    for (const Part& p : parts) memcpy(static_cast<char*>(host) + p.off, p.src, p.bytes);
   }
 };
-
-template <class T>
-int ensure_for(DevBuf& d, const std::vector<T>& v) {
-  QB_CUDA(d.ensure(std::max<size_t>(v.size() * sizeof(T), 16)));
-  return QB_OK;
-}
 
 int batch_loop(qb_handle* h, const qb_problem* problems, const std::vector<int32_t>& ids, const qb_options* o,
                qb_result* r) {
@@ -1139,17 +1133,18 @@ int batch_run(qb_handle* h, const qb_problem* problems, const std::vector<int32_
   const int m = (int)ids.size();
   if (!m) return QB_OK;
   std::vector<qb::BatchInst> insts(m);
-  // every problem's W, then the tensor-core problems' scaled W, packed in pinned memory
+  // every problem's W, packed in pinned memory
   uint64_t w_total = 0;
   for (int j = 0; j < m; ++j) w_total += (uint64_t)problems[ids[j]].n * problems[ids[j]].n;
-  QB_CUDA(h->hbat.ensure(2 * w_total * sizeof(double) + 64));
+  const bool graph = (o->flags & QB_FLAG_GRAPH) != 0;
+  DevBuf* B = h->bat;
+  QB_CUDA(h->hbat.ensure(w_total * sizeof(double) + 64));
+  QB_CUDA(B[0].ensure(std::max<uint64_t>(w_total, 2) * sizeof(double)));
   double* Wall = static_cast<double*>(h->hbat.p);
-  double* Wtc = Wall + w_total;
-  uint64_t w_used = 0, wtc_used = 0;
   std::vector<qb::BatchItem> gitems, uitems;
   std::vector<uint32_t> gray_ids;  // problems with a selection step (Gray and tensor-core forms)
   std::vector<qb::BatchCand> pre;
-  std::vector<std::pair<int, uint64_t>> tcs;  // (problem, offset in Wtc)
+  std::vector<int> tcs;  // the tensor-core problems
   uint64_t gtab_total = 0, rec_total = 0;
   size_t sm_gtab = 0, sm_gray = 0, sm_exact = 0;
   int n_tc_max = 0;
@@ -1161,6 +1156,26 @@ int batch_run(qb_handle* h, const qb_problem* problems, const std::vector<int32_
   std::vector<double> sums(m, 0.0);
   std::vector<char> ints(m, 0);
   std::vector<int> rcs(m, QB_OK);
+  // the 16-bit pair kernel's unit, offset and bound for each problem it would run, where it fits
+  struct PairFit {
+    bool fits = false;
+    double sigma = 1.0, eps = 0.0;
+    float dmin = 0.f;
+  };
+  std::vector<PairFit> fit(m);
+  auto tc_form = [&](int n, bool is_int) {
+    const qb_handle::Tuned& T = h->tuned[is_int ? 1 : 0][n];
+    // the tuned form of (dtype class, n) when qb_autotune chose one, else tensor-core from 24
+    return tc_allowed && qb::tc_supported(n) && (T.form ? T.form == QB_FORM_TC : n >= kBatchTcMinN);
+  };
+  auto pair_fit = [&](int j) {
+    const int n = problems[ids[j]].n;
+    if (rcs[j] || !tc_form(n, ints[j] != 0)) return;
+    const double* W = Wall + w_offs[j];
+    const bool digits = ints[j] && sums[j] <= qb::kTcIntMaxAbsSum;
+    fit[j].fits = (digits && qb::tc2_u16_eligible(n, W, &fit[j].dmin)) ||
+                  qb::tc2_u16_quantized(n, W, sums[j], &fit[j].sigma, &fit[j].dmin, &fit[j].eps);
+  };
   {
     uint64_t off = 0;
     for (int j = 0; j < m; ++j) {
@@ -1175,6 +1190,7 @@ int batch_run(qb_handle* h, const qb_problem* problems, const std::vector<int32_
       rcs[j] = load_problem(h, p, Wv, &sums[j], &ii);
       ints[j] = ii;
       if (!rcs[j]) memcpy(Wall + w_offs[j], Wv.data(), Wv.size() * sizeof(double));
+      pair_fit(j);
     }
     auto convert = [&](int j0, int j1) {
       for (int j = j0; j < j1; ++j) {
@@ -1183,34 +1199,42 @@ int batch_run(qb_handle* h, const qb_problem* problems, const std::vector<int32_
         bool ii = false;
         rcs[j] = load_host_problem_into(p, Wall + w_offs[j], &sums[j], &ii);
         ints[j] = ii;
+        pair_fit(j);
       }
     };
-    parallel_ranges(m, convert);
+    parallel_ranges(m, w_total, convert);
   }
-  std::vector<std::pair<int, double>> tc_scale;  // (problem, scale) of the tensor-core problems
+  for (int j = 0; j < m; ++j) {
+    if (rcs[j]) return rcs[j];
+    if (sums[j] >= kTwo53) return QB_ERANGE;
+    if (o->prefix_bits > problems[ids[j]].n) return QB_EINVAL;
+  }
+  // launch by launch, W travels while the host plans; an early return waits for it
+  struct CopyGuard {
+    cudaStream_t st;
+    bool armed;
+    ~CopyGuard() {
+      if (armed) cudaStreamSynchronize(st);
+    }
+  } guard{h->st, !graph};
+  if (!graph)
+    QB_CUDA(cudaMemcpyAsync(B[0].p, Wall, w_total * sizeof(double), cudaMemcpyHostToDevice, h->st));
   for (int j = 0; j < m; ++j) {
     const qb_problem* p = &problems[ids[j]];
     const int n = p->n;
     const double abs_sum = sums[j];
     const bool is_int = ints[j] != 0;
-    if (rcs[j]) return rcs[j];
-    if (abs_sum >= kTwo53) return QB_ERANGE;
     qb::BatchInst& I = insts[j];
     memset(&I, 0, sizeof(I));
     I.n = n;
     I.is_int = is_int ? 1 : 0;
     I.natural = o->tie_rule == QB_TIE_NATURAL ? 1 : 0;
     I.A = o->prefix_bits < 0 ? n - std::min(n, 20) : o->prefix_bits;
-    if (I.A > n) return QB_EINVAL;
     I.B = n - I.A;
     I.w_off = w_offs[j];
-    w_used += (uint64_t)n * n;
     int free_bits;
     const qb_handle::Tuned& T = h->tuned[is_int ? 1 : 0][n];
-    // the tuned form of (dtype class, n) when qb_autotune chose one, else tensor-core from 24
-    const bool use_tc = tc_allowed && qb::tc_supported(n) &&
-                        (T.form ? T.form == QB_FORM_TC : n >= kBatchTcMinN);
-    if (use_tc) {
+    if (tc_form(n, is_int)) {
       qb::TcPlan tp;
       qb::tc_plan(n, is_int, abs_sum, 0, 1, &tp, T.tc_gl);
       I.kind = qb::kBatchTC;
@@ -1221,9 +1245,7 @@ int batch_run(qb_handle* h, const qb_problem* problems, const std::vector<int32_
       I.eps = tp.eps;
       I.rec_off = rec_total;
       rec_total += I.nrec;
-      tcs.emplace_back(j, wtc_used);
-      tc_scale.emplace_back(j, tp.scale);
-      wtc_used += (uint64_t)n * n;
+      tcs.push_back(j);
       gray_ids.push_back((uint32_t)j);
       n_tc_max = std::max(n_tc_max, n);
       free_bits = I.gl + 12;
@@ -1265,82 +1287,53 @@ int batch_run(qb_handle* h, const qb_problem* problems, const std::vector<int32_
   // problem's eps; each problem gets a table of its 16-bit constants.
   std::vector<qb::Tc2Tab> tc_tabs;
   bool tc_pair = !tcs.empty() && !(o->flags & (QB_FLAG_TC_ONE | QB_FLAG_TC_NO16));
-  if (tc_pair) {
-    tc_tabs.resize(tcs.size());
-    std::vector<double> sg(tcs.size(), 1.0), ep(tcs.size(), 0.0);
-    for (size_t k = 0; k < tcs.size() && tc_pair; ++k) {
-      const int j = tcs[k].first;
-      const int n = insts[j].n;
-      const double* W = Wall + w_offs[j];
-      float dm = 0.f;
-      const bool fits = (insts[j].exact_digits && qb::tc2_u16_eligible(n, W, &dm)) ||
-                        qb::tc2_u16_quantized(n, W, sums[j], &sg[k], &dm, &ep[k]);
-      if (!fits) {
-        tc_pair = false;
-        break;
-      }
-      float gamma[8];
-      for (int b = 0; b < 8; ++b) gamma[b] = (float)(W[(size_t)(n - 16) * n + (n - 1 - b)] * sg[k]);
-      qb::tc2_u16_tables(gamma, dm, &tc_tabs[k]);
-    }
-    if (tc_pair) {  // every member fits: only now change the members' plans
-      for (size_t k = 0; k < tcs.size(); ++k) {
-        qb::BatchInst& I = insts[tcs[k].first];
-        if (ep[k] > 0.0) I.exact_digits = 0;  // rounded values (the digits flag is unused by this kernel)
-        I.scale = sg[k];
-        I.eps = ep[k];
-        I.tc_kernel = 4;
-        tc_scale[k].second = sg[k];
-      }
-    } else {
-      tc_tabs.clear();
-    }
+  for (int j : tcs) tc_pair = tc_pair && fit[j].fits;
+  if (tc_pair) tc_tabs.resize(tcs.size());
+  for (size_t k = 0; k < tcs.size(); ++k) {
+    const int j = tcs[k];
+    qb::BatchInst& I = insts[j];
+    I.tc_kernel = tc_pair ? 4 : 1;
+    if (!tc_pair) continue;
+    const PairFit& F = fit[j];
+    if (F.eps > 0.0) I.exact_digits = 0;  // rounded values (the digits flag is unused by this kernel)
+    I.scale = F.sigma;
+    I.eps = F.eps;
+    const double* W = Wall + w_offs[j];
+    float gamma[8];
+    for (int b = 0; b < 8; ++b) gamma[b] = (float)(W[(size_t)(I.n - 16) * I.n + (I.n - 1 - b)] * F.sigma);
+    qb::tc2_u16_tables(gamma, F.dmin, &tc_tabs[k]);
   }
-  for (auto& t : tcs)
-    if (!insts[t.first].tc_kernel) insts[t.first].tc_kernel = 1;
-  // the tensor-core problems' W scaled into their own block (several threads)
-  parallel_ranges((int)tcs.size(), [&](int k0, int k1) {
-    for (int k = k0; k < k1; ++k) {
-      const int j = tcs[k].first;
-      const uint64_t nn = (uint64_t)insts[j].n * insts[j].n;
-      const double sc = tc_scale[k].second;
-      const double* W = Wall + w_offs[j];
-      double* dst = Wtc + tcs[k].second;
-      for (uint64_t e = 0; e < nn; ++e) dst[e] = W[e] * sc;
-    }
-  });
   // candidate list: the small problems' records first, then room for the Gray problems'
   const int prefilled = (int)pre.size();
   const int cap = prefilled + std::max(4096, 8 * (int)gray_ids.size());
-  DevBuf* B = h->bat;
   int rc;
   // the tensor-core problems' record blocks, dealt out as contiguous runs to one persistent
   // CTA per SM (a run may span problems: one item per problem piece)
   std::vector<qb::TcItem> items;
   std::vector<qb::Tc2Tab> item_tabs;                 // the 16-bit pair kernel: per item
-  std::vector<std::pair<uint64_t, uint64_t>> offs;  // (scaled-W offset, record offset) per item
+  std::vector<std::pair<uint64_t, uint64_t>> offs;  // (W offset, record offset) per item
   std::vector<uint32_t> first(1, 0);
   if (!tcs.empty()) {
     uint64_t total = 0;
-    for (auto& t : tcs) total += 1ull << (insts[t.first].n - 15 - insts[t.first].gl);
+    for (int j : tcs) total += 1ull << (insts[j].n - 15 - insts[j].gl);
     const uint64_t ctas = std::min<uint64_t>((uint64_t)h->sm_count, total);
     const uint64_t per = (total + ctas - 1) / ctas;
     uint64_t left = per;
     for (size_t k = 0; k < tcs.size(); ++k) {
-      const auto& t = tcs[k];
-      const qb::BatchInst& I = insts[t.first];
+      const qb::BatchInst& I = insts[tcs[k]];
       const uint64_t groups = 1ull << (I.n - 15 - I.gl);
       uint64_t g = 0;
       while (g < groups) {
         const uint64_t take = std::min(left, groups - g);
         qb::TcItem it{};
-        offs.emplace_back(t.second, I.rec_off + (g << 3));
+        offs.emplace_back(I.w_off, I.rec_off + (g << 3));
         it.i_begin = g << I.gl;
         it.ntiles = take << I.gl;
         it.n = I.n;
         it.gl = I.gl;
         it.exact = I.exact_digits;
         it.inv_scale = (float)(1.0 / I.scale);
+        it.scale = I.scale;
         items.push_back(it);
         if (tc_pair) item_tabs.push_back(tc_tabs[k]);
         g += take;
@@ -1353,63 +1346,50 @@ int batch_run(qb_handle* h, const qb_problem* problems, const std::vector<int32_
     }
     if (first.back() != (uint32_t)items.size()) first.push_back((uint32_t)items.size());
   }
-  // every device and pinned host allocation happens here, before any copy or launch is issued
-  QB_CUDA(B[0].ensure(std::max<uint64_t>(w_used, 2) * sizeof(double)));
-  if ((rc = ensure_for(B[1], insts))) return rc;
-  if ((rc = ensure_for(B[2], gitems))) return rc;
-  if ((rc = ensure_for(B[3], uitems))) return rc;
-  if ((rc = ensure_for(B[4], gray_ids))) return rc;
-  QB_CUDA(B[5].ensure((size_t)cap * sizeof(qb::BatchCand)));
+  // one block for the results, copied in at its initial values with the rest and copied back:
+  // emin[m], kmin[m] (uint64), pass1_min[m] (float), candidate count, the tensor-core kernel's
+  // error word, the exact kernel's next item
+  const size_t mb = (size_t)m * 8;
+  const size_t res_bytes = 2 * mb + (size_t)m * 4 + 3 * sizeof(int);
+  Arena ar;
+  const size_t off_inst = ar.add(insts), off_git = ar.add(gitems), off_uit = ar.add(uitems), off_gid = ar.add(gray_ids);
+  const size_t off_item = ar.add(items), off_first = ar.add(first), off_tab = ar.add(item_tabs);
+  const size_t off_res = ar.add_raw(nullptr, res_bytes);
+  const size_t off_cand = ar.add(pre);  // last: the candidates' room reaches on from here
+  // every device and pinned host allocation happens here
+  QB_CUDA(B[1].ensure(off_cand + (size_t)cap * sizeof(qb::BatchCand)));
   QB_CUDA(B[6].ensure((size_t)cap * sizeof(qb::ExactOut)));
   QB_CUDA(B[7].ensure(std::max<uint64_t>(gtab_total, 4) * sizeof(float)));
   QB_CUDA(B[8].ensure(std::max<uint64_t>(rec_total, 4) * sizeof(float)));
-  // minima: emin[m], kmin[m] (uint64), pass1_min[m] (float), cand_count (int)
-  const size_t mb = (size_t)m * 8;
-  const size_t res_bytes = 2 * mb + (size_t)m * 4 + sizeof(int);
-  QB_CUDA(B[9].ensure(res_bytes + 16));
-  if (!tcs.empty()) {
-    QB_CUDA(B[10].ensure(std::max<uint64_t>(wtc_used, 2) * sizeof(double)));
-    if ((rc = ensure_for(B[11], items))) return rc;
-    if ((rc = ensure_for(B[12], first))) return rc;
-    QB_CUDA(B[13].ensure(16));
-    if (tc_pair && (rc = ensure_for(B[14], item_tabs))) return rc;
-  }
-  QB_CUDA(h->hout.ensure(res_bytes + 16));
-  uint64_t* emin = static_cast<uint64_t*>(B[9].p);
-  uint64_t* kmin = emin + m;
-  float* p1min = reinterpret_cast<float*>(kmin + m);
-  int* ccount = reinterpret_cast<int*>(static_cast<char*>(B[9].p) + 2 * mb + (size_t)m * 4);
+  QB_CUDA(h->hout.ensure(res_bytes));
+  QB_CUDA(h->hstage.ensure(ar.size));
+  char* dar = static_cast<char*>(B[1].p);
+  char* har = static_cast<char*>(h->hstage.p);
   for (size_t k = 0; k < items.size(); ++k) {  // device addresses of the items' W and records
-    items[k].W = static_cast<const double*>(B[10].p) + offs[k].first;
+    items[k].W = static_cast<const double*>(B[0].p) + offs[k].first;
     items[k].rec = static_cast<float*>(B[8].p) + offs[k].second;
   }
-  Stage stg;
-  stg.add(B[1].p, insts);
-  stg.add(B[2].p, gitems);
-  stg.add(B[3].p, uitems);
-  stg.add(B[4].p, gray_ids);
-  stg.add(B[5].p, pre);
-  stg.add(ccount, std::vector<int>(1, prefilled));
-  if (!tcs.empty()) {
-    stg.add(B[11].p, items);
-    stg.add(B[12].p, first);
-    if (tc_pair) stg.add(B[14].p, item_tabs);
-  }
-  QB_CUDA(h->hstage.ensure(std::max<size_t>(stg.bytes.size(), 16)));
-  memcpy(h->hstage.p, stg.bytes.data(), stg.bytes.size());
-  int64_t h2d_bytes = (int64_t)(w_used * sizeof(double)) + (int64_t)(wtc_used * sizeof(double));
-  for (auto& c : stg.copies) h2d_bytes += (int64_t)c.bytes;
-  unsigned* tc_err = tcs.empty() ? nullptr : static_cast<unsigned*>(B[13].p);
-  const int64_t d2h_bytes = (int64_t)res_bytes + (tc_err ? (int64_t)sizeof(unsigned) : 0);
+  ar.fill(har);
+  memset(har + off_res, 0xff, 2 * mb);
+  memset(har + off_res + 2 * mb, 0, res_bytes - 2 * mb);
+  *reinterpret_cast<int*>(har + off_res + 2 * mb + (size_t)m * 4) = prefilled;
+  uint64_t* emin = reinterpret_cast<uint64_t*>(dar + off_res);
+  uint64_t* kmin = emin + m;
+  float* p1min = reinterpret_cast<float*>(kmin + m);
+  int* ccount = reinterpret_cast<int*>(p1min + m);
+  unsigned* tc_err = reinterpret_cast<unsigned*>(ccount + 1);
+  unsigned* next = tc_err + 1;
+  const int64_t h2d_bytes = (int64_t)(w_total * sizeof(double)) + (int64_t)ar.size;
+  const int64_t d2h_bytes = (int64_t)res_bytes;
   const double* dW = static_cast<const double*>(B[0].p);
-  const qb::BatchInst* dI = static_cast<const qb::BatchInst*>(B[1].p);
-  qb::BatchCand* dC = static_cast<qb::BatchCand*>(B[5].p);
+  const qb::BatchInst* dI = reinterpret_cast<const qb::BatchInst*>(dar + off_inst);
+  qb::BatchCand* dC = reinterpret_cast<qb::BatchCand*>(dar + off_cand);
   qb::ExactOut* dO = static_cast<qb::ExactOut*>(B[6].p);
   qb::TcParams P{};
   size_t sm_tc = 0;
   if (!tcs.empty()) {
-    P.items = static_cast<const qb::TcItem*>(B[11].p);
-    P.item_first = static_cast<const uint32_t*>(B[12].p);
+    P.items = reinterpret_cast<const qb::TcItem*>(dar + off_item);
+    P.item_first = reinterpret_cast<const uint32_t*>(dar + off_first);
     P.n_max = n_tc_max;
     P.err = tc_err;
     const qb::TcSmemLayout L = qb::tc_layout(n_tc_max);
@@ -1423,76 +1403,60 @@ int batch_run(qb_handle* h, const qb_problem* problems, const std::vector<int32_
   }
   const unsigned key_blocks = (unsigned)std::min<int>((cap + 255) / 256, h->sm_count * 4);
 
-  // the whole device side of the batch: uploads, the six launches, the result copy
+  // the exact kernel's CTAs take candidates in turn: as many as run at once, if there are that many
+  const unsigned exact_blocks = (unsigned)std::min<int>(cap, 2 * h->sm_count);
+
+  // the whole device side of the batch: uploads, the launches, the result copy
   auto issue = [&](cudaStream_t st, bool timed) -> int {
-    QB_CUDA(cudaMemcpyAsync(B[0].p, Wall, w_used * sizeof(double), cudaMemcpyHostToDevice, st));
-    for (auto& c : stg.copies)
-      QB_CUDA(cudaMemcpyAsync(c.dst, static_cast<unsigned char*>(h->hstage.p) + c.off, c.bytes,
-                              cudaMemcpyHostToDevice, st));
-    QB_CUDA(cudaMemsetAsync(B[9].p, 0xff, 2 * mb, st));
-    if (timed) {
-      QB_CUDA(cudaEventRecord(h->ev[0], st));
-      QB_CUDA(cudaEventRecord(h->ev[4], st));
-    }
+    if (graph) QB_CUDA(cudaMemcpyAsync(B[0].p, Wall, w_total * sizeof(double), cudaMemcpyHostToDevice, st));
+    QB_CUDA(cudaMemcpyAsync(dar, har, ar.size, cudaMemcpyHostToDevice, st));
+    if (timed) QB_CUDA(cudaEventRecord(h->ev[0], st));
     if (any_gray) {
       qb::batch_gtab_kernel<<<(unsigned)gitems.size(), 256, sm_gtab, st>>>(
-          dI, static_cast<const qb::BatchItem*>(B[2].p), dW, static_cast<float*>(B[7].p));
+          dI, reinterpret_cast<const qb::BatchItem*>(dar + off_git), dW, static_cast<float*>(B[7].p));
       qb::batch_gray_kernel<<<(unsigned)uitems.size(), qb::kGrayThreads, sm_gray, st>>>(
-          dI, static_cast<const qb::BatchItem*>(B[3].p), dW, static_cast<const float*>(B[7].p),
+          dI, reinterpret_cast<const qb::BatchItem*>(dar + off_uit), dW, static_cast<const float*>(B[7].p),
           static_cast<float*>(B[8].p));
       h->kernels += 2;
     }
     if (!tcs.empty()) {
-      QB_CUDA(cudaMemcpyAsync(B[10].p, Wtc, wtc_used * sizeof(double), cudaMemcpyHostToDevice, st));
-      QB_CUDA(cudaMemsetAsync(tc_err, 0, 16, st));
       if (tc_pair) {
         qb::Tc2Params Q2{};
         Q2.P = P;
-        Q2.tabs = static_cast<const qb::Tc2Tab*>(B[14].p);
+        Q2.tabs = reinterpret_cast<const qb::Tc2Tab*>(dar + off_tab);
         qb::tc_pair_kernel<true><<<(unsigned)(first.size() - 1), qb::kTc2Threads, sm_tc, st>>>(Q2);
       } else
         qb::tc_pass1_kernel<true><<<(unsigned)(first.size() - 1), qb::kTcThreads, sm_tc, st>>>(P);
       ++h->kernels;
     }
-    if (timed) {
-      QB_CUDA(cudaEventRecord(h->ev[5], st));
-      QB_CUDA(cudaEventRecord(h->ev[1], st));
-      QB_CUDA(cudaEventRecord(h->ev[2], st));
-    }
+    if (timed) QB_CUDA(cudaEventRecord(h->ev[1], st));
     if (!gray_ids.empty()) {
       qb::batch_select_kernel<<<(unsigned)gray_ids.size(), 256, 0, st>>>(
-          dI, static_cast<const uint32_t*>(B[4].p), static_cast<const float*>(B[8].p), dC, ccount, cap, p1min,
-          emin, kmin);
+          dI, reinterpret_cast<const uint32_t*>(dar + off_gid), static_cast<const float*>(B[8].p), dC, ccount, cap,
+          p1min, emin, kmin);
       ++h->kernels;
     }
-    qb::batch_exact_kernel<<<(unsigned)cap, qb::kExactThreads, sm_exact, st>>>(dI, dW, dC, ccount, cap, dO, emin);
+    qb::batch_exact_kernel<<<exact_blocks, qb::kExactThreads, sm_exact, st>>>(dI, dW, dC, ccount, cap, next, dO, emin);
     qb::batch_key_kernel<<<key_blocks, 256, 0, st>>>(dC, ccount, cap, dO, emin, kmin);
     h->kernels += 2;
     QB_CUDA(cudaGetLastError());
     if (timed) QB_CUDA(cudaEventRecord(h->ev[3], st));
-    QB_CUDA(cudaMemcpyAsync(h->hout.p, B[9].p, res_bytes, cudaMemcpyDeviceToHost, st));
-    if (tc_err)
-      QB_CUDA(cudaMemcpyAsync(static_cast<char*>(h->hout.p) + res_bytes, tc_err, sizeof(unsigned),
-                              cudaMemcpyDeviceToHost, st));
+    QB_CUDA(cudaMemcpyAsync(h->hout.p, emin, res_bytes, cudaMemcpyDeviceToHost, st));
     return QB_OK;
   };
 
-  const bool graph = (o->flags & QB_FLAG_GRAPH) != 0;
   if (graph) {
     // one graph launch per batch; the graph is captured again whenever the batch's shape, the
     // options or any buffer address differ from the captured one
-    std::vector<uint64_t> key = {(uint64_t)m, (uint64_t)w_used, (uint64_t)wtc_used, (uint64_t)cap,
+    std::vector<uint64_t> key = {(uint64_t)m, (uint64_t)w_total, (uint64_t)ar.size, (uint64_t)cap,
                                  (uint64_t)gitems.size(), (uint64_t)uitems.size(), (uint64_t)gray_ids.size(),
                                  (uint64_t)first.size(), (uint64_t)sm_gtab, (uint64_t)sm_gray, (uint64_t)sm_exact,
                                  (uint64_t)sm_tc, (uint64_t)any_gray, (uint64_t)tc_pair, (uint64_t)(uintptr_t)Wall,
                                  (uint64_t)(uintptr_t)h->hstage.p, (uint64_t)(uintptr_t)h->hout.p,
                                  (uint64_t)(uintptr_t)h->own};
-    for (int k = 0; k < 14; ++k) key.push_back((uint64_t)(uintptr_t)B[k].p);
-    for (auto& c : stg.copies) {
-      key.push_back((uint64_t)(uintptr_t)c.dst);
-      key.push_back((uint64_t)c.off);
-      key.push_back((uint64_t)c.bytes);
-    }
+    for (int k : {0, 1, 6, 7, 8}) key.push_back((uint64_t)(uintptr_t)B[k].p);
+    for (size_t off : {off_inst, off_git, off_uit, off_gid, off_item, off_first, off_tab, off_res, off_cand})
+      key.push_back((uint64_t)off);
     if (!h->batch_graph || key != h->batch_graph_key) {
       if (h->batch_graph) {
         cudaGraphExecDestroy(h->batch_graph);
@@ -1528,15 +1492,12 @@ int batch_run(qb_handle* h, const qb_problem* problems, const std::vector<int32_
   h->h2d += h2d_bytes;
   h->d2h += d2h_bytes;
   QB_CUDA(cudaStreamSynchronize(h->st));
+  guard.armed = false;
   const uint64_t* he = static_cast<const uint64_t*>(h->hout.p);
   const uint64_t* hk = he + m;
   const float* hp = reinterpret_cast<const float*>(hk + m);
-  const int got = *reinterpret_cast<const int*>(reinterpret_cast<const char*>(h->hout.p) + 2 * mb + (size_t)m * 4);
-  if (tc_err) {
-    unsigned e = 0;
-    memcpy(&e, static_cast<const char*>(h->hout.p) + res_bytes, sizeof(unsigned));
-    if (e & qb::kErrTimeout) return QB_ETIMEOUT;
-  }
+  const int got = *reinterpret_cast<const int*>(hp + m);
+  if (reinterpret_cast<const unsigned*>(hp + m)[1] & qb::kErrTimeout) return QB_ETIMEOUT;
   if (got > cap) {
     *overflow = true;
     return QB_OK;
@@ -1547,8 +1508,8 @@ int batch_run(qb_handle* h, const qb_problem* problems, const std::vector<int32_
     km = p1;
   } else {
     QB_CUDA(cudaEventElapsedTime(&p1, h->ev[0], h->ev[1]));
-    QB_CUDA(cudaEventElapsedTime(&p2, h->ev[2], h->ev[3]));
-    QB_CUDA(cudaEventElapsedTime(&km, h->ev[4], h->ev[5]));
+    QB_CUDA(cudaEventElapsedTime(&p2, h->ev[1], h->ev[3]));
+    km = p1;
   }
   for (int j = 0; j < m; ++j) {
     const qb::BatchInst& I = insts[j];

@@ -127,12 +127,13 @@ inline bool tc_u16_eligible(int n, const double* W, float* dmin, double* span = 
 
 // one CTA work item: a contiguous run of whole record blocks of one problem
 struct TcItem {
-  const double* W;     // scaled W of the problem, n*n
+  const double* W;     // W of the problem, n*n
   float* rec;          // record 0 of the item's first block
   uint64_t i_begin;    // Gray index of the item's first tile (a multiple of 2^gl)
   uint64_t ntiles;     // tiles in the item (a multiple of 2^gl, below 2^31)
   int n, gl, exact;
-  float inv_scale;     // 1 / scale of W
+  float inv_scale;     // 1 / scale
+  double scale;        // power of two applied to W as it is loaded
 };
 
 struct TcParams {
@@ -140,7 +141,8 @@ struct TcParams {
   int stall;
   int exact;
   float inv_scale;
-  const double* W;          // scaled W, n*n
+  double scale;             // power of two applied to W as it is loaded
+  const double* W;          // W, n*n
   uint64_t tile_begin;      // shard start (aligned to 2^gl)
   uint64_t groups;          // record blocks (2^gl tiles each) in this shard
   uint64_t groups_per_cta;  // contiguous blocks per CTA (last CTA may have fewer)
@@ -466,7 +468,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_pass1_kernel(TcParams P) {
     if (g0 >= P.groups) return;  // uniform per CTA
     const uint64_t g1 = min(P.groups, g0 + P.groups_per_cta);
     one = TcItem{P.W, P.rec + (g0 << 3), P.tile_begin + (g0 << P.gl), (g1 - g0) << P.gl, P.n, P.gl, P.exact,
-                 P.inv_scale};
+                 P.inv_scale, P.scale};
   }
 
   // ---------------------------------------------------------------- one-time set-up
@@ -514,7 +516,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_pass1_kernel(TcParams P) {
       *reinterpret_cast<float**>(tc_smem + L.misc_off + 16) = rec;
       *reinterpret_cast<float*>(tc_smem + L.misc_off + 24) = inv_scale;
     }
-    for (int i = tid; i < n * n; i += kTcThreads) Ws[i] = I.W[i];
+    for (int i = tid; i < n * n; i += kTcThreads) Ws[i] = I.W[i] * I.scale;
     // the item's records start at +inf (the epilogue folds into them with atomic minima)
     for (uint64_t r = (uint64_t)tid; r < ((ntiles >> gl) << 3); r += kTcThreads) rec[r] = __int_as_float(0x7f800000);
     __syncthreads();
@@ -895,8 +897,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_pass1_kernel(TcParams P) {
 }
 
 // the search kernel itself (one persistent CTA per SM)
-// Wsc: W times the plan's scale; err: the error word (cleared)
-inline int tc_launch(const TcPlan& p, float* rec, const double* Wsc, unsigned* err, cudaStream_t st, int sms,
+// W: n*n on the device; err: the error word (cleared)
+inline int tc_launch(const TcPlan& p, float* rec, const double* W, unsigned* err, cudaStream_t st, int sms,
                      int* kernels) {
   const uint64_t groups = (p.tile_end - p.tile_begin) >> p.gl;
   if (!groups) return 0;
@@ -910,7 +912,8 @@ inline int tc_launch(const TcPlan& p, float* rec, const double* Wsc, unsigned* e
   P.gl = p.gl;
   P.exact = p.exact ? 1 : 0;
   P.inv_scale = (float)(1.0 / p.scale);
-  P.W = Wsc;
+  P.W = W;
+  P.scale = p.scale;
   P.tile_begin = p.tile_begin;
   P.groups = groups;
   P.groups_per_cta = gpc;

@@ -412,7 +412,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_pair_fp32_kernel(const __gri
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tmem_slot)));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
-  for (int i = tid; i < n * n; i += kTcThreads) Ws[i] = P.W[i];
+  for (int i = tid; i < n * n; i += kTcThreads) Ws[i] = P.W[i] * P.scale;
   for (uint64_t r = (uint64_t)tid; r < ((ntiles >> gl) << 3); r += kTcThreads) rec[r] = __int_as_float(0x7f800000);
   __syncthreads();
   // A operand (constant)
@@ -729,8 +729,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_pair_fp32_kernel(const __gri
 // in uniform registers), warps 4-19 the epilogue.  Between a batch's items all roles meet at a
 // CTA barrier with the pipelines empty (every MMA has been waited for by its epilogue warps),
 // so the per-item tables, B operand columns and constants can be rewritten; barrier slots, B
-// stages and phases follow the CTA-wide block counter bbase.  W is in the problem's units
-// (scaled by sigma off the exact path).
+// stages and phases follow the CTA-wide block counter bbase.  W is taken in the
+// problem's units (times scale as it is loaded: sigma off the exact path).
 //
 // What bounds it: the epilogue's ALU work.  Per warp and 8192 states 72 packed minima and 2
 // float minima of 88 ALU instructions (half rate: 176 of the measured 225 cycles per scheduler,
@@ -789,14 +789,14 @@ __global__ void __launch_bounds__(kTc2Threads, 1) tc_pair_kernel(const __grid_co
     if (g0 >= P.groups) return;  // uniform per CTA
     const uint64_t g1 = min(P.groups, g0 + P.groups_per_cta);
     one = TcItem{P.W, P.rec + (g0 << 3), P.tile_begin + (g0 << P.gl), (g1 - g0) << P.gl, P.n, P.gl, P.exact,
-                 P.inv_scale};
+                 P.inv_scale, P.scale};
   }
 
   // the item's W into shared memory, its records to +infinity, its corrections
   auto load_item = [&](uint32_t it) {
     const TcItem I = kItems ? P.items[it] : one;
     const Tc2Tab& Tb = kItems ? Q.tabs[it] : Q.tab;
-    for (int i = tid; i < I.n * I.n; i += kTc2Threads) Ws[i] = I.W[i];
+    for (int i = tid; i < I.n * I.n; i += kTc2Threads) Ws[i] = I.W[i] * I.scale;
     for (uint64_t r = (uint64_t)tid; r < ((I.ntiles >> I.gl) << 3); r += kTc2Threads) I.rec[r] = __int_as_float(0x7f800000);
     if (tid < 24) Ct[tid] = tid < 8 ? Tb.corr_t[0][tid] : Tb.corr_p[0][(tid - 8) >> 3][tid & 7];
   };
@@ -1241,9 +1241,9 @@ __global__ void __launch_bounds__(kTc2Threads, 1) tc_pair_kernel(const __grid_co
 
 // the pair-form search kernel (one persistent CTA per SM); gamma = couplings of variable
 // n-16 with u bits 0..7, in the units of the scaled W
-// Wsc: W times the plan's scale; err: the error word (cleared); min_key: receives the smallest
+// W: n*n on the device; err: the error word (cleared); min_key: receives the smallest
 // record value (16-bit form; initially 0xffffffff)
-inline int tc2_launch(const TcPlan& p, const float* gamma, float* rec, const double* Wsc, unsigned* err,
+inline int tc2_launch(const TcPlan& p, const float* gamma, float* rec, const double* W, unsigned* err,
                       uint32_t* min_key, cudaStream_t st, int sms, int* kernels) {
   const uint64_t groups = (p.tile_end - p.tile_begin) >> p.gl;
   if (!groups) return 0;
@@ -1258,7 +1258,8 @@ inline int tc2_launch(const TcPlan& p, const float* gamma, float* rec, const dou
   P.gl = p.gl;
   P.exact = p.exact ? 1 : 0;
   P.inv_scale = (float)(1.0 / p.scale);
-  P.W = Wsc;
+  P.W = W;
+  P.scale = p.scale;
   P.tile_begin = p.tile_begin;
   P.groups = groups;
   P.groups_per_cta = gpc;
