@@ -74,6 +74,9 @@ class QbError(RuntimeError):
         super().__init__(f"{where}: {strerror(status)} (status {status})")
 
 
+_DTYPE_IDS = {id(d): code for d, code in _DTYPES.items()}  # numpy's native dtype objects are singletons
+_PROBLEM_DTYPE = np.dtype(QbProblem)
+
 _lib = None
 _lock = threading.Lock()
 
@@ -221,28 +224,38 @@ class Handle:
         outlive the call that reads them)."""
         count = len(Qs)
         probs = (QbProblem * count)()
-        keep = [Q if (isinstance(Q, np.ndarray) and Q.flags.c_contiguous) else np.ascontiguousarray(Q) for Q in Qs]
-        nl, cl, pl = [0] * count, [0] * count, [0] * count
-        for i, Q in enumerate(keep):
-            sh = Q.shape
-            if len(sh) != 2 or sh[0] != sh[1]:
-                raise ValueError(f"Q must be square, got shape {sh}")
-            code = _DTYPES.get(Q.dtype)
-            if code is None:
-                raise TypeError(f"unsupported Q dtype {Q.dtype}")
-            nl[i] = sh[0]
-            cl[i] = code
-            # the data address: through the buffer protocol for writable non-empty arrays (a
-            # third of the cost of building __array_interface__), else the interface dict
-            pl[i] = _addressof(_char_from_buffer(Q)) if (sh[0] and Q.flags.writeable) else Q.__array_interface__["data"][0]
-        ns = np.array(nl, dtype=np.int64)
+        # the data addresses through the buffer protocol (a third of the cost of building
+        # __array_interface__), which refuses what is not writable, C-contiguous and non-empty:
+        # then one by one
+        addr = None
+        keep = list(Qs)
+        if set(map(type, keep)) == {np.ndarray}:
+            try:
+                addr = [_addressof(_char_from_buffer(Q)) for Q in keep]
+            except (TypeError, ValueError, BufferError):
+                pass
+        if addr is None:
+            keep = [Q if (isinstance(Q, np.ndarray) and Q.flags.c_contiguous) else np.ascontiguousarray(Q) for Q in Qs]
+        shapes = [Q.shape for Q in keep]
+        ns = np.zeros(count, dtype=np.int64)
         if count:
+            for sh in set(shapes):
+                if len(sh) != 2 or sh[0] != sh[1]:
+                    raise ValueError(f"Q must be square, got shape {sh}")
+            ns[:] = [sh[0] for sh in shapes]
+            codes = [_DTYPE_IDS.get(id(Q.dtype)) for Q in keep]
+            if None in codes:  # dtype objects other than numpy's own native ones
+                codes = [_DTYPES.get(Q.dtype) for Q in keep]
+                if None in codes:
+                    raise TypeError(f"unsupported Q dtype {keep[codes.index(None)].dtype}")
+            if addr is None:
+                addr = [Q.__array_interface__["data"][0] for Q in keep]
             # the problem descriptors filled column by column through a structured view
-            view = np.frombuffer(probs, dtype=np.dtype(QbProblem))
+            view = np.frombuffer(probs, dtype=_PROBLEM_DTYPE)
             view["n"] = ns
             view["ldq"] = ns
-            view["dtype"] = cl
-            view["q"] = pl
+            view["dtype"] = codes
+            view["q"] = addr
         return probs, ns, keep
 
     def solve_batch(self, Qs: list, **opts) -> "BatchResults":

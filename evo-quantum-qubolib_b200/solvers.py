@@ -50,12 +50,17 @@ logger = logging.getLogger(__name__)
 ALL_METRICS = {"time_arr", "energy_arr"}
 
 
-def _torch_stream(device: int):
+def _current_stream(device: int):
+    """The torch stream current on ``device``, which becomes the current device."""
     import torch
     if not torch.cuda.is_available():
         raise RuntimeError("qubo_b200 needs a CUDA device; torch.cuda.is_available() is False")
     torch.cuda.set_device(device)
-    return torch.cuda.current_stream(device).cuda_stream
+    return torch.cuda.current_stream(device)
+
+
+def _torch_stream(device: int):
+    return _current_stream(device).cuda_stream
 
 
 _json_pool = None
@@ -149,12 +154,13 @@ class QBF(SolverABC):
         self.check_obsolete_args(**kwargs)
         self.kwargs = kwargs
         dev = self.parse_device_arg(**kwargs)
-        stream = _torch_stream(dev)
-        self.timer = PerformanceTimer(use_gpu=True)
+        current = _current_stream(dev)
+        stream = current.cuda_stream
+        self.timer = PerformanceTimer(use_gpu=True, stream=current)
         self.N = problem.N
         Q = np.asarray(problem.build_Q_matrix(use_gpu=False))
         self.Q = Q
-        self.timer.pick_time("build_Q")
+        self.timer.mark_time("build_Q")
         self.A, self.B = QBF.define_chunk_size(N=self.N, size_of=Q.dtype.itemsize, **kwargs)
         if self.A < 0 or self.B < 1 or self.A + self.B != self.N:
             raise ValueError(f"invalid split A={self.A}, B={self.B} for N={self.N}")
@@ -179,10 +185,11 @@ class QBF(SolverABC):
         self.kwargs = kwargs
         self.json_str = _json.encode(kwargs, indent=4)
         dev = self.parse_device_arg(**kwargs)
-        stream = _torch_stream(dev)
-        self.timer = PerformanceTimer(use_gpu=True)
+        current = _current_stream(dev)
+        stream = current.cuda_stream
+        self.timer = PerformanceTimer(use_gpu=True, stream=current)
         Qs = [np.asarray(p.build_Q_matrix(use_gpu=False)) for p in problems]
-        self.timer.pick_time("build_Q")
+        self.timer.mark_time("build_Q")
         results = _lib.handle(dev).solve_batch(Qs, form=kwargs.get("form", "auto"), tie_rule="qbf", fixed_bits=0,
                                                prefix_bits=int(kwargs.get("A", -1)), stream=stream,
                                                graph=bool(kwargs.get("graph", False)))
@@ -249,8 +256,9 @@ class QB_F1(SolverABC):
     def solve(self, problem: ProblemABC, **kwargs) -> Solution:
         self.check_obsolete_args(**kwargs)
         dev = self.parse_device_arg(**kwargs)
-        stream = _torch_stream(dev)
-        self.timer = PerformanceTimer(use_gpu=True)
+        current = _current_stream(dev)
+        stream = current.cuda_stream
+        self.timer = PerformanceTimer(use_gpu=True, stream=current)
         self.N = problem.N
         self.B = 18
         self.A = self.N - self.B
@@ -260,7 +268,7 @@ class QB_F1(SolverABC):
         if self.A < 1:
             raise ValueError(f"QB_F1 needs N >= 19 (B is fixed to 18), got N={self.N}")
         self.Q = Q
-        self.timer.pick_time("build_Q")
+        self.timer.mark_time("build_Q")
         wrap = bool(kwargs.get("int16_wrap", False))
         enc = _encode_async(problem, kwargs, Q)  # submitted last: it runs during the device search
         res = _lib.handle(dev).solve(Q, form=kwargs.get("form", "auto"), tie_rule="qb_f1", fixed_bits=0,
