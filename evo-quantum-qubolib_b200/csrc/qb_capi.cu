@@ -948,7 +948,7 @@ int qbf1_wrap_solve(qb_handle* h, const qb_problem* p, const qb_options* o, qb_r
   QB_CUDA(B[0].ensure(Qi.size() * sizeof(int)));
   QB_CUDA(B[6].ensure(cols * sizeof(short)));
   QB_CUDA(B[7].ensure((size_t)A * cols * sizeof(short)));
-  QB_CUDA(B[8].ensure(steps * sizeof(short)));
+  QB_CUDA(B[8].ensure(steps * sizeof(uint32_t)));
   constexpr size_t key_bytes = qb::kQbf1Threads * sizeof(unsigned long long);
   QB_CUDA(B[9].ensure(key_bytes + sizeof(qb::Qbf1Answer)));
   QB_CUDA(cudaMemcpyAsync(B[0].p, Qi.data(), Qi.size() * sizeof(int), cudaMemcpyHostToDevice, h->st));
@@ -956,26 +956,25 @@ int qbf1_wrap_solve(qb_handle* h, const qb_problem* p, const qb_options* o, qb_r
   const int* dQ = static_cast<const int*>(B[0].p);
   short* BB = static_cast<short*>(B[6].p);
   short* ABBA = static_cast<short*>(B[7].p);
-  short* AA = static_cast<short*>(B[8].p);
+  uint32_t* AA = static_cast<uint32_t*>(B[8].p);
   unsigned long long* key = static_cast<unsigned long long*>(B[9].p);
   qb::Qbf1Answer* ans = reinterpret_cast<qb::Qbf1Answer*>(key + qb::kQbf1Threads);
   QB_CUDA(cudaMemsetAsync(key, 0xff, key_bytes + sizeof(qb::Qbf1Answer), h->st));
   QB_CUDA(cudaEventRecord(h->ev[0], h->st));
   const size_t smt = qb::qbf1w_tables_smem(n, A);
-  qb::qbf1w_tables_kernel<<<1u << (qb::kQbf1B - qb::kQbf1Lo), 256, smt, h->st>>>(dQ, n, A, BB, ABBA);
-  qb::qbf1w_prefix_kernel<<<(unsigned)std::min<uint64_t>((steps + 255) / 256, (uint64_t)h->sm_count * 8), 256,
-                            (size_t)A * A * sizeof(int), h->st>>>(dQ, n, A, AA);
+  const unsigned prefix_blocks = (unsigned)std::min<uint64_t>((steps + 255) / 256, (uint64_t)h->sm_count * 8);
+  qb::qbf1w_tables_kernel<<<qb::kQbf1TableBlocks + prefix_blocks, 256, smt, h->st>>>(dQ, n, A, BB, ABBA, AA);
   const uint64_t nchunks = std::min<uint64_t>(64, std::max<uint64_t>(4, steps));
   const uint64_t chunk_len = (steps + nchunks - 1) / nchunks;
   const size_t sm = qb::qbf1w_search_smem(A);
   QB_CUDA(cudaEventRecord(h->ev[4], h->st));
-  qb::qbf1w_search_kernel<<<dim3(qb::kQbf1Threads / 64, (unsigned)(nchunks / 4)), 256, sm, h->st>>>(
+  qb::qbf1w_search_kernel<<<dim3(qb::kQbf1Threads / 64, (unsigned)((nchunks + 7) / 8)), 256, sm, h->st>>>(
       A, BB, ABBA, AA, chunk_len, key);
   QB_CUDA(cudaEventRecord(h->ev[5], h->st));
   // the winning thread, its exact step and that prefix's suffix, then one copy back
   qb::qbf1w_final_kernel<<<1, 512, 0, h->st>>>(A, BB, ABBA, AA, key, qb::qbf1w_group(chunk_len), ans);
   qb::qbf1w_row_kernel<<<(unsigned)(cols / 256), 256, 0, h->st>>>(A, BB, ABBA, ans);
-  h->kernels += 5;
+  h->kernels += 4;
   QB_CUDA(cudaGetLastError());
   QB_CUDA(cudaEventRecord(h->ev[1], h->st));
   static_assert(sizeof(qb::Qbf1Answer) <= 64, "hmisc");

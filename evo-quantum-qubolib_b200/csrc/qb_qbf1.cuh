@@ -23,26 +23,70 @@ constexpr int kQbf1MaxN = 46;
 
 __device__ __forceinline__ int wrap16(int v) { return (int)(short)v; }
 
-// BB[s] and ABBA[k][s] (k < A) for every 18-bit suffix s (MSB-first: bit 17 - j of s is
-// variable A + j).  Q: n x n int32 copy of the int16 matrix.  One block per value of the upper 9
-// suffix bits, whose sums (for BB, for every row k and for the fields of the lower 9 variables)
-// its threads share; a thread adds the lower bits' for two neighbouring suffixes.  8 us at
-// A = 16, against 32 us with every suffix summed alone.
+// The tables, one launch.  Blocks 0 .. 511: BB[s] and ABBA[k][s] (k < A) for every 18-bit suffix s
+// (MSB-first: bit 17 - j of s is variable A + j), one block per value of the upper 9 suffix bits,
+// whose sums (for BB, for every row k and for the fields of the lower 9 variables) its threads
+// share; a thread adds the lower bits' for two neighbouring suffixes.  The other blocks: AA[i] =
+// int16 of E_pre(gray(i)) (prefix bit A-1-k is variable k) in both halves of a word, 256 steps at
+// a time, whose upper bits' sums are shared the same way.  Q: n x n int32 copy of the int16 matrix.
+// A = 16: 11.7 us, against 11.7 + 9.4 us as two kernels with every prefix summed alone.
 constexpr int kQbf1Lo = 9;
+constexpr int kQbf1TableBlocks = 1 << (kQbf1B - kQbf1Lo);
 inline size_t qbf1w_tables_smem(int n, int A) {
   return ((size_t)n * n + (size_t)A * (kQbf1Lo + 1) + kQbf1Lo * kQbf1Lo + kQbf1Lo + 1) * sizeof(int);
 }
+__device__ inline void qbf1w_prefix(const int* q, int n, int A, uint32_t* __restrict__ AA, int* sm) {
+  int* lw = sm;        // [b][c]: couplings among the 8 lowest prefix bits, diagonal W_bb
+  int* f = lw + 64;    // [b]: their fields from the upper bits; [8]: the upper bits' energy
+  const int t = threadIdx.x, lane = t & 31;
+  auto W = [&](int u, int v) { return u == v ? q[u * n + u] : q[u * n + v] + q[v * n + u]; };
+  if (t < 64) lw[t] = (t >> 3) < A && (t & 7) < A ? W(A - 1 - (t >> 3), A - 1 - (t & 7)) : 0;
+  const uint64_t steps = 1ull << A;
+  const int nh = A - 8;  // upper bits: bit m is variable nh - 1 - m
+  for (uint64_t g = blockIdx.x - kQbf1TableBlocks; (g << 8) < steps; g += gridDim.x - kQbf1TableBlocks) {
+    const uint64_t hi = gray64(g);
+    if (t < 64) {  // warp 0: the fields; warp 1: the energy, a bit per lane
+      int v = 0;
+      const int own = t < 32 ? (lane < 8 ? A - 1 - lane : -1) : (lane < nh && ((hi >> lane) & 1) ? nh - 1 - lane : -1);
+      if (own >= 0) {
+        if (t >= 32) v = W(own, own);
+        for (int m = 0; m < (t < 32 ? nh : lane); ++m)
+          if ((hi >> m) & 1) v += W(own, nh - 1 - m);
+      }
+      if (t >= 32) v = __reduce_add_sync(0xffffffffu, v);
+      if (t < 8 || t == 32) f[t < 8 ? t : 8] = v;
+    }
+    __syncthreads();
+    const uint64_t i = (g << 8) + (uint64_t)t;
+    const int p = (int)(gray64(i) & 255ull);
+    int e = f[8];
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+      int r = lw[b * 8 + b] + f[b];
+#pragma unroll
+      for (int c = 0; c < b; ++c) r += ((p >> c) & 1) ? lw[b * 8 + c] : 0;
+      e += ((p >> b) & 1) ? r : 0;
+    }
+    if (i < steps) AA[i] = ((uint32_t)e & 0xffffu) * 0x10001u;
+    __syncthreads();
+  }
+}
 __global__ void __launch_bounds__(256) qbf1w_tables_kernel(const int* __restrict__ Q, int n, int A,
-                                                           short* __restrict__ BB, short* __restrict__ ABBA) {
-  extern __shared__ int q1_smem[];
+                                                           short* __restrict__ BB, short* __restrict__ ABBA,
+                                                           uint32_t* __restrict__ AA) {
+  extern __shared__ __align__(16) int q1_smem[];
+  const int t = threadIdx.x;
+  for (int i = t; i < n * n; i += blockDim.x) q1_smem[i] = Q[i];
+  __syncthreads();
+  if (blockIdx.x >= kQbf1TableBlocks) {  // uniform per block
+    qbf1w_prefix(q1_smem, n, A, AA, q1_smem + n * n);
+    return;
+  }
   int* clo = q1_smem + n * n;            // [k][b]: couplings of row k with lower suffix bit b
   int* slo = clo + A * kQbf1Lo;          // [b][c]: couplings among the lower bits, diagonal W_bb
   int* chi = slo + kQbf1Lo * kQbf1Lo;    // [k]: row k's sum over the block's upper bits
   int* fhi = chi + A;                    // [b]: lower bit b's field from the upper bits; [9]: their energy
-  const int t = threadIdx.x;
   const int hi = blockIdx.x;             // suffix bits 9 .. 17
-  for (int i = t; i < n * n; i += blockDim.x) q1_smem[i] = Q[i];
-  __syncthreads();
   auto W = [&](int u, int v) { return u == v ? q1_smem[u * n + u] : q1_smem[u * n + v] + q1_smem[v * n + u]; };
   const int v0 = n - 1;                  // variable of suffix bit 0; bit b: v0 - b
   for (int i = t; i < A * kQbf1Lo; i += blockDim.x) clo[i] = W(i / kQbf1Lo, v0 - i % kQbf1Lo);
@@ -85,24 +129,6 @@ __global__ void __launch_bounds__(256) qbf1w_tables_kernel(const int* __restrict
   }
 }
 
-// AA[i] = int16 of E_pre(gray(i)) (prefix bit A-1-k is variable k)
-__global__ void qbf1w_prefix_kernel(const int* __restrict__ Q, int n, int A, short* __restrict__ AA) {
-  extern __shared__ int q1p_smem[];
-  for (int i = threadIdx.x; i < A * A; i += blockDim.x) q1p_smem[i] = Q[(i / A) * n + (i % A)];
-  __syncthreads();
-  const uint64_t steps = 1ull << A;
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < steps; i += (uint64_t)gridDim.x * blockDim.x) {
-    const uint64_t p = gray64(i);
-    int e = 0;
-    for (int k = 0; k < A; ++k) {
-      if (!((p >> (A - 1 - k)) & 1)) continue;
-      for (int l = 0; l < A; ++l)
-        if ((p >> (A - 1 - l)) & 1) e += q1p_smem[k * A + l];
-    }
-    AA[i] = (short)wrap16(e);
-  }
-}
-
 // packed int16 pairs: per-halfword add (wraps modulo 2^16) and signed minimum
 __device__ __forceinline__ uint32_t add16x2(uint32_t x, uint32_t y) {
   uint32_t r;
@@ -114,7 +140,24 @@ __device__ __forceinline__ uint32_t min16x2(uint32_t x, uint32_t y) {
   asm("min.s16x2 %0, %1, %2;" : "=r"(r) : "r"(x), "r"(y));
   return r;
 }
-__device__ __forceinline__ uint32_t pack16(int lo, int hi) { return (uint32_t)(uint16_t)lo | ((uint32_t)(uint16_t)hi << 16); }
+// per halfword -x
+__device__ __forceinline__ uint32_t neg16x2(uint32_t x) { return add16x2(~x, 0x00010001u); }
+
+// signed minimum of 16 packed pairs
+__device__ __forceinline__ uint32_t min16x2_16(const uint32_t* e) {
+  const uint32_t a = __vimin3_s16x2(__vimin3_s16x2(e[0], e[1], e[2]), e[3], e[4]);
+  const uint32_t b = __vimin3_s16x2(__vimin3_s16x2(e[5], e[6], e[7]), e[8], e[9]);
+  const uint32_t c = __vimin3_s16x2(__vimin3_s16x2(e[10], e[11], e[12]), e[13], e[14]);
+  return min16x2(__vimin3_s16x2(a, b, c), e[15]);
+}
+
+// signed minimum of 16 packed sums e + r, each wrapping modulo 2^16 (fused add-and-minimum)
+__device__ __forceinline__ uint32_t addmin16x2_16(const uint32_t* e, const uint32_t* r) {
+  uint32_t m = add16x2(e[0], r[0]);
+#pragma unroll
+  for (int c = 1; c < 16; ++c) m = __viaddmin_s16x2(e[c], r[c], m);
+  return m;
+}
 
 // shared memory of the search kernel: +ABBA and -ABBA rows of the block's 1024 columns,
 // two columns per 32-bit word
@@ -124,137 +167,128 @@ inline size_t qbf1w_search_smem(int A) { return (size_t)2 * A * 512 * sizeof(uin
 // and reports the group of its best step, a shorter one the step itself
 __host__ __device__ inline int qbf1w_group(uint64_t chunk_len) { return (chunk_len & 31) == 0 ? 32 : 1; }
 
-// signed minimum of 8 packed pairs
-__device__ __forceinline__ uint32_t min16x2_8(const uint32_t* e) {
-  return __vimin3_s16x2(__vimin3_s16x2(e[0], e[1], e[2]), __vimin3_s16x2(e[3], e[4], e[5]), min16x2(e[6], e[7]));
-}
-
-// The search.  blockIdx.x = the reference block (64 threads, 1024 columns), blockIdx.y picks
-// 4 consecutive chunks of Gray steps; thread = (chunk lane, reference thread t).  Thread t's
-// 16 columns 64 c + t are held as 8 int16 pairs (c = 2 c2, 2 c2 + 1), so one step costs 8
-// packed adds and 4 three-input packed minima; a step that turns a prefix variable off adds the
-// negated row.  Chunks of at least 32 steps are walked in aligned groups of 32 unrolled steps,
-// in which the flipped prefix bit and its direction are constants; the rows of the two lowest
-// prefix bits (three steps of four) stay in registers.  Two steps' minima over their columns are
-// packed into one word (even step low), which one add.u16x2 with the packed AA entries turns
-// into both steps' values, wrapping like the reference's int16; a group keeps only its minimum,
-// and the exact step is found afterwards for the one thread that wins (qbf1w_final_kernel).
-// Each thread reports (best int16 value, its group) of its chunk into key[tid] by a 64-bit
-// atomic min, which keeps the smallest value and, among equal values, the earliest group.
+// The search.  blockIdx.x = the reference block (64 threads, 1024 columns); a warp walks one chunk
+// of Gray steps (8 per CTA, blockIdx.y) for all of the block's threads: lane l has the reference
+// threads 2 l and 2 l + 1 in the halves of its words, word c their columns 64 c + t.  A step's
+// minimum over the 16 columns is thus 16 packed values and needs no merging of halves before the
+// AA entry is added.  Chunks of at least 32 steps are walked in aligned groups of 32, in which the
+// flipped prefix bit and its direction are constants.  The words hold the state without prefix
+// bits 0 and 1: four steps in a row share it, their minima are those of E, F = E + r0, F + r1 and
+// E + r1 (rows in registers; a Gray group of four visits them in either direction), the last two
+// by fused add-and-minimum without storing the sums, and only every fourth step updates the words
+// (with the negated row where a variable is turned off).  All sums wrap like the reference's
+// int16.  A group keeps only its minimum, and the exact step is found afterwards for the one
+// thread that wins (qbf1w_final_kernel).  Each thread reports (best int16 value, its group) of
+// its chunk into key[tid] by a 64-bit atomic min, which keeps the smallest value and, among equal
+// values, the earliest group.
 //
-// What bounds it: the register reads and the half-rate pipes of the 8 adds (FMA pipe) and 5.75
-// minima and permutes (ALU) per step of 16 states.  2^34 states (n = 34): 727 us, against
-// 1230 us with one step at a time (44 instructions per step: the halves extracted, added and
-// compared as scalars, every row read from shared memory).
-__global__ void __launch_bounds__(256, 3) qbf1w_search_kernel(int A, const short* __restrict__ BB,
+// What bounds it: the half-rate packed pipes (per step 13.8 ALU and 9.2 FMA-pipe instructions of 32
+// states a lane: 72% and 48% of what they can take) with the register reads of the three-operand
+// forms beside them.  2^34 states (n = 34): 565 us; all sums of two steps of four by fused
+// add-and-minimum, F not stored, 575 us (80% of the ALU).  With a reference thread's column pairs
+// in a word, every step's sums stored and the halves merged per step it was 722 us.
+__global__ void __launch_bounds__(256, 2) qbf1w_search_kernel(int A, const short* __restrict__ BB,
                                                               const short* __restrict__ ABBA,
-                                                              const short* __restrict__ AA, uint64_t chunk_len,
+                                                              const uint32_t* __restrict__ AA, uint64_t chunk_len,
                                                               unsigned long long* __restrict__ key) {
-  extern __shared__ uint32_t q1w_smem[];  // [2][A][8][64]: word (row k, pair c2, thread t)
+  extern __shared__ __align__(16) uint32_t q1w_smem[];  // [2][A][16][32]: word (row k, column index c, lane)
   const int blk = blockIdx.x;
-  for (int i = threadIdx.x; i < A * 512; i += blockDim.x) {
-    const int k = i >> 9, c2 = (i >> 6) & 7, tt = i & 63;
-    const size_t base = (size_t)k * (1 << kQbf1B) + (size_t)blk * 1024 + tt;
-    const int lo = ABBA[base + 64 * (2 * c2)], hi = ABBA[base + 64 * (2 * c2 + 1)];
-    q1w_smem[i] = pack16(lo, hi);
-    q1w_smem[A * 512 + i] = pack16(-lo, -hi);
+  for (int i = threadIdx.x; i < A * 128; i += blockDim.x) {
+    const uint4 w = reinterpret_cast<const uint4*>(ABBA + ((size_t)(i >> 7) << kQbf1B) + (size_t)blk * 1024)[i & 127];
+    reinterpret_cast<uint4*>(q1w_smem)[i] = w;
+    reinterpret_cast<uint4*>(q1w_smem)[A * 128 + i] =
+        make_uint4(neg16x2(w.x), neg16x2(w.y), neg16x2(w.z), neg16x2(w.w));
   }
   __syncthreads();
-  const int t = threadIdx.x & 63;
-  const uint64_t chunk = (uint64_t)blockIdx.y * 4 + (threadIdx.x >> 6);
+  const int lane = threadIdx.x & 31;
+  const uint64_t chunk = (uint64_t)blockIdx.y * 8 + (threadIdx.x >> 5);
   const uint64_t steps = 1ull << A;
   const uint64_t i0 = chunk * chunk_len;
   if (i0 >= steps) return;
   const uint64_t i1 = min(steps, i0 + chunk_len);
-  const uint32_t* pos = q1w_smem + t;            // + row * 512 + c2 * 64
-  const uint32_t* neg = q1w_smem + A * 512 + t;
-  uint32_t E2[8];
+  const uint32_t* pos = q1w_smem + lane;            // + row * 512 + c * 32
+  const uint32_t* neg = q1w_smem + A * 512 + lane;
+  uint32_t E2[16];
   {
     const uint64_t p0 = gray64(i0);
+    const uint32_t* b = reinterpret_cast<const uint32_t*>(BB) + blk * 512 + lane;
 #pragma unroll
-    for (int c2 = 0; c2 < 8; ++c2) E2[c2] = pack16(BB[blk * 1024 + 128 * c2 + t], BB[blk * 1024 + 128 * c2 + 64 + t]);
+    for (int c = 0; c < 16; ++c) E2[c] = b[c * 32];
     for (int k = 0; k < A; ++k)
       if ((p0 >> (A - 1 - k)) & 1) {
 #pragma unroll
-        for (int c2 = 0; c2 < 8; ++c2) E2[c2] = add16x2(E2[c2], pos[k * 512 + c2 * 64]);
+        for (int c = 0; c < 16; ++c) E2[c] = add16x2(E2[c], pos[k * 512 + c * 32]);
       }
   }
-  int best;
-  uint64_t bi = i0;
+  int best[2];
+  uint64_t bi[2] = {i0, i0};
   if ((chunk_len & 31) == 0) {
-    best = 32768;  // above every int16
-    uint32_t lp[2][2][8];  // rows of prefix bits 0 and 1 (variables A-1, A-2), on and off
+    best[0] = best[1] = 32768;  // above every int16
+    uint32_t r0[16], r1[16];  // rows of prefix bits 0 and 1 (variables A-1, A-2)
 #pragma unroll
-    for (int kb = 0; kb < 2; ++kb)
-#pragma unroll
-      for (int c2 = 0; c2 < 8; ++c2) {
-        lp[kb][0][c2] = pos[(A - 1 - kb) * 512 + c2 * 64];
-        lp[kb][1][c2] = neg[(A - 1 - kb) * 512 + c2 * 64];
-      }
+    for (int c = 0; c < 16; ++c) {
+      r0[c] = pos[(A - 1) * 512 + c * 32];
+      r1[c] = pos[(A - 2) * 512 + c * 32];
+    }
     for (uint64_t ig = i0; ig < i1; ig += 32) {
-      uint32_t aa[16];  // AA[ig .. ig + 31], two per word
-      {
-        const uint4* src = reinterpret_cast<const uint4*>(AA + ig);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const uint4 w = __ldg(src + q);
-          aa[4 * q] = w.x;
-          aa[4 * q + 1] = w.y;
-          aa[4 * q + 2] = w.z;
-          aa[4 * q + 3] = w.w;
-        }
-      }
+      const uint4* aa = reinterpret_cast<const uint4*>(AA + ig);
       if (ig != i0) {  // the chunk's first step is its start state
         const int kb = __ffsll((long long)ig) - 1;  // >= 5
         const uint32_t* r = (((gray64(ig) >> kb) & 1) ? pos : neg) + (A - 1 - kb) * 512;
 #pragma unroll
-        for (int c2 = 0; c2 < 8; ++c2) E2[c2] = add16x2(E2[c2], r[c2 * 64]);
+        for (int c = 0; c < 16; ++c) E2[c] = add16x2(E2[c], r[c * 32]);
       }
       const uint32_t* r4 = (((ig >> 5) & 1) ? neg : pos) + (A - 5) * 512;  // prefix bit 4: off in odd groups
-      uint32_t gm = 0u;
+      uint32_t gm = 0x7fff7fffu;
 #pragma unroll
-      for (int l = 0; l < 32; l += 2) {
-        if (l) {
-          const int kb = ctz5(l);  // >= 1
-          const bool on = !((l >> (kb + 1)) & 1);
+      for (int q = 0; q < 8; ++q) {  // four steps each
+        const uint4 a = __ldg(aa + q);
+        if (q) {
+          const int kb = 2 + ctz5(q);
+          const bool on = !((q >> (kb - 1)) & 1);
           const uint32_t* r = kb == 4 ? r4 : (on ? pos : neg) + (A - 1 - kb) * 512;
 #pragma unroll
-          for (int c2 = 0; c2 < 8; ++c2) E2[c2] = add16x2(E2[c2], kb == 1 ? lp[1][on ? 0 : 1][c2] : r[c2 * 64]);
+          for (int c = 0; c < 16; ++c) E2[c] = add16x2(E2[c], r[c * 32]);
         }
-        const uint32_t m0 = min16x2_8(E2);
+        // prefix bits (1, 0): 00, 01, 11, 10 where prefix bit 2 was last 0, else the reverse
+        uint32_t F2[16];
 #pragma unroll
-        for (int c2 = 0; c2 < 8; ++c2) E2[c2] = add16x2(E2[c2], lp[0][(l >> 1) & 1][c2]);
-        const uint32_t m1 = min16x2_8(E2);
-        const uint32_t tt = add16x2(min16x2(__byte_perm(m0, m1, 0x5410), __byte_perm(m0, m1, 0x7632)), aa[l >> 1]);
-        gm = l ? min16x2(gm, tt) : tt;
+        for (int c = 0; c < 16; ++c) F2[c] = add16x2(E2[c], r0[c]);
+        const uint32_t m00 = min16x2_16(E2), m01 = min16x2_16(F2), m11 = addmin16x2_16(F2, r1),
+                       m10 = addmin16x2_16(E2, r1);
+        gm = __vimin3_s16x2(gm, add16x2(m00, q & 1 ? a.w : a.x), add16x2(m01, q & 1 ? a.z : a.y));
+        gm = __vimin3_s16x2(gm, add16x2(m11, q & 1 ? a.y : a.z), add16x2(m10, q & 1 ? a.x : a.w));
       }
-      const int g = min((int)(short)(gm & 0xffffu), (int)gm >> 16);
-      if (g < best) {  // strict: the earliest group keeps a tie
-        best = g;
-        bi = ig;
-      }
+      const int g[2] = {(int)(short)(gm & 0xffffu), (int)gm >> 16};
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        if (g[h] < best[h]) {  // strict: the earliest group keeps a tie
+          best[h] = g[h];
+          bi[h] = ig;
+        }
     }
   } else {
-    auto step_min = [&]() -> int {
-      const uint32_t m2 = min16x2_8(E2);
-      return min((int)(short)(m2 & 0xffffu), (int)m2 >> 16);
-    };
-    best = wrap16((int)AA[i0] + step_min());
-    for (uint64_t i = i0 + 1; i < i1; ++i) {
-      const int kb = __ffsll((long long)i) - 1;
-      const bool on = (gray64(i) >> kb) & 1;
-      const uint32_t* r = (on ? pos : neg) + (A - 1 - kb) * 512;
+    best[0] = best[1] = 32768;
+    for (uint64_t i = i0; i < i1; ++i) {
+      if (i != i0) {
+        const int kb = __ffsll((long long)i) - 1;
+        const uint32_t* r = (((gray64(i) >> kb) & 1) ? pos : neg) + (A - 1 - kb) * 512;
 #pragma unroll
-      for (int c2 = 0; c2 < 8; ++c2) E2[c2] = add16x2(E2[c2], r[c2 * 64]);
-      const int tt = wrap16((int)AA[i] + step_min());
-      if (tt < best) {
-        best = tt;
-        bi = i;
+        for (int c = 0; c < 16; ++c) E2[c] = add16x2(E2[c], r[c * 32]);
       }
+      const uint32_t tt = add16x2(min16x2_16(E2), AA[i]);
+      const int g[2] = {(int)(short)(tt & 0xffffu), (int)tt >> 16};
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        if (g[h] < best[h]) {
+          best[h] = g[h];
+          bi[h] = i;
+        }
     }
   }
-  const int tid = blk * 64 + t;
-  atomicMin(key + tid, ((unsigned long long)(best + 32768) << 40) | (unsigned long long)bi);
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+    atomicMin(key + blk * 64 + 2 * lane + h, ((unsigned long long)(best[h] + 32768) << 40) | (unsigned long long)bi[h]);
 }
 
 // The answer's parts, on the device: what the reference's host picks from the threads' results.
@@ -269,7 +303,7 @@ struct Qbf1Answer {
 // first step of its reported group with that value: warp c evaluates the thread's column c at the
 // group's 32 steps from the tables.
 __global__ void __launch_bounds__(512) qbf1w_final_kernel(int A, const short* __restrict__ BB,
-                                                          const short* __restrict__ ABBA, const short* __restrict__ AA,
+                                                          const short* __restrict__ ABBA, const uint32_t* __restrict__ AA,
                                                           const unsigned long long* __restrict__ key, int group,
                                                           Qbf1Answer* __restrict__ ans) {
   __shared__ unsigned long long red[16];
@@ -303,15 +337,18 @@ __global__ void __launch_bounds__(512) qbf1w_final_kernel(int A, const short* __
     const int col = (tid >> 6) * 1024 + 64 * warp + (tid & 63);
     const uint64_t p = gray64(st);
     v = BB[col];
-    for (int k = 0; k < A; ++k)
-      if ((p >> (A - 1 - k)) & 1) v += ABBA[(size_t)k * (1 << kQbf1B) + col];
+#pragma unroll 8
+    for (int k = 0; k < A; ++k) {
+      const int w = ABBA[((size_t)k << kQbf1B) + col];
+      v += ((p >> (A - 1 - k)) & 1) ? w : 0;
+    }
     v = wrap16(v);
   }
   val[warp][lane] = v;
   __syncthreads();
   if (warp == 0) {
     for (int c = 1; c < 16; ++c) v = min(v, val[c][lane]);
-    const bool hit = in && wrap16((int)AA[in ? st : s0] + v) == best16;
+    const bool hit = in && wrap16((int)(short)AA[in ? st : s0] + v) == best16;
     const unsigned h = __ballot_sync(0xffffffffu, hit);
     if (lane == 0) {
       ans->step = s0 + (uint64_t)(h ? __ffs(h) - 1 : 0);
