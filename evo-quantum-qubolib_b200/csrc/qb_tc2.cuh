@@ -11,7 +11,7 @@
 // One MMA computes D for tile t; the epilogue reads each accumulator once and derives the
 // partner tile's value from it.  Every TMEM accumulator thus stands for two states, which
 // halves the MMAs, accumulator round trips and TMEM loads per state.  Measured on B200
-// (n = 36 TSP QUBO, 2^36 states): fp32 pair form 3.83 ms, 16-bit pair form (below) 1.72 ms,
+// (n = 36 TSP QUBO, 2^36 states): fp32 pair form 3.83 ms, 16-bit pair form (below) 1.75 ms,
 // against 3.8-3.95 ms for one state per accumulator; the 16-bit pair form is the default
 // where it applies, and qb_autotune times both forms.
 //
@@ -736,7 +736,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_pair_fp32_kernel(const __gri
 // float minima of 88 ALU instructions (half rate: 176 of the measured 225 cycles per scheduler,
 // 0.78 busy); register reads (about 1.8 operands per cycle and scheduler) allow the 16
 // corrections and the row terms beside them, but not one more add per register.  Measured
-// (n = 36, 2^36 states, the kernel alone): 1.72 ms, against 2.36 ms with one B stage and one
+// (n = 36, 2^36 states, the kernel alone): 1.75 ms (1.72-1.77 between cards), against 2.36 ms with one B stage and one
 // N = 256 MMA per pair, issued by one thread of a divergent warp.  On the way: the low t bits
 // in the A operand with one MMA issuer 2.66; uniform MMA issue 2.33; two issuers and the
 // epilogue's four pairs per block unrolled 2.03; waits without a result register, u16 -> f32
@@ -747,7 +747,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_pair_fp32_kernel(const __gri
 // cycles against 196 from TMEM, the register read ports), each group issuing its own MMA
 // behind a named barrier (2.37), three groups on a ring of four accumulators (2.33), one N =
 // 256 MMA per pair (2.03 at the 2.00 stage), 3.5 instead of 4 minima per 8 inputs by moving
-// the odd input behind the correction (1.80 against 1.75).
+// the odd input behind the correction (1.80 against 1.75), corrections as constant operands
+// (1.83-1.90), two groups of four warps with two accumulators each and the next unit's load in
+// flight (12 warps, 165 registers: 2.01-2.09), row terms inside the MMA so that corrections and
+// conversions run once per block (1.79: its second K slice costs what they save).
 template <bool kItems>
 __global__ void __launch_bounds__(kTc2Threads, 1) tc_pair_kernel(const __grid_constant__ Tc2Params Q) {
   constexpr int KW = kTc2Low, NS = 1 << KW;  // low t bits per block, pairs per block
