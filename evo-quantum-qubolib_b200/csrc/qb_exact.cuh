@@ -215,11 +215,19 @@ __device__ __forceinline__ ExactOut exact_record_min(const ProblemDev& P, const 
   __syncthreads();
   // the tables of the thread's start, of the register patterns and of the walk steps
   if (warp == 0) {
-    double e = 0.0;
+    // the fields' sum counts every coupling twice: halved as a whole it stays a whole number for
+    // integer W (single fields' halves would not, and FP64 holds halves only below 2^52)
+    double e = 0.0, h = 0.0;
     for (int v = lane; v < n; v += 32)
-      if ((base >> (n - 1 - v)) & 1) e += Ws[v * n + v] + 0.5 * hs[v];
-    for (int off = 16; off; off >>= 1) e += __shfl_xor_sync(0xffffffffu, e, off);
-    if (lane == 0) e_base = e;
+      if ((base >> (n - 1 - v)) & 1) {
+        e += Ws[v * n + v];
+        h += hs[v];
+      }
+    for (int off = 16; off; off >>= 1) {
+      e += __shfl_xor_sync(0xffffffffu, e, off);
+      h += __shfl_xor_sync(0xffffffffu, h, off);
+    }
+    if (lane == 0) e_base = e + 0.5 * h;
   } else if (warp == 1) {
     double s = 0.0;  // register pattern g = lane
 #pragma unroll
