@@ -111,7 +111,7 @@ def _text(o, pad: str, step: str) -> str:
         if not o:
             return "[]"
         return f"[\n{inner}" + f",\n{inner}".join([_text(v, inner, step) for v in o]) + f"\n{pad}]"
-    elif isinstance(o, (np.generic, type, tuple, set, frozenset, dict, list, str, int, float)) or \
+    elif isinstance(o, (np.ndarray, np.generic, type, tuple, set, frozenset, dict, list, str, int, float)) or \
             getattr(o, "__dict__", None) is None:
         # the rarer kinds, and any subclass of the ones above, by the standard encoder
         return json.dumps(_enc(o), indent=len(step)).replace("\n", "\n" + pad)
