@@ -106,7 +106,8 @@ def _text(o, pad: str, step: str) -> str:
         return (f'{{\n{inner}"py/numpy.ndarray": {{\n{deep}"dtype": {d},\n{deep}"shape": {shape},\n{deep}"b64": "{data}"'
                 f"\n{inner}}}\n{pad}}}")
     if t is dict:
-        items = [f"{_quote(str(k))}: {_text(v, inner, step)}" for k, v in o.items()]
+        texts = {str(k): v for k, v in o.items()}  # keys of equal text: one entry, the last value
+        items = [f"{_quote(k)}: {_text(v, inner, step)}" for k, v in texts.items()]
     elif t is list:
         if not o:
             return "[]"
