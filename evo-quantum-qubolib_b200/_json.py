@@ -78,7 +78,6 @@ def _dec(o):
 
 
 _quote = json.encoder.encode_basestring_ascii
-_DTYPE_STR = {}  # dtype -> its quoted string
 
 
 def _text(o, pad: str, step: str) -> str:
@@ -96,14 +95,11 @@ def _text(o, pad: str, step: str) -> str:
         return int.__repr__(o)
     inner = pad + step
     if t is np.ndarray:
-        d = _DTYPE_STR.get(o.dtype)
-        if d is None:
-            d = _DTYPE_STR[o.dtype] = _quote(o.dtype.str)
         deep = inner + step
         dims = f",\n{deep}{step}".join(map(str, o.shape))
         shape = f"[\n{deep}{step}{dims}\n{deep}]" if o.shape else "[]"
         data = base64.b64encode(np.ascontiguousarray(o).tobytes()).decode()
-        return (f'{{\n{inner}"py/numpy.ndarray": {{\n{deep}"dtype": {d},\n{deep}"shape": {shape},\n{deep}"b64": "{data}"'
+        return (f'{{\n{inner}"py/numpy.ndarray": {{\n{deep}"dtype": {_quote(o.dtype.str)},\n{deep}"shape": {shape},\n{deep}"b64": "{data}"'
                 f"\n{inner}}}\n{pad}}}")
     if t is dict:
         texts = {str(k): v for k, v in o.items()}  # keys of equal text: one entry, the last value
