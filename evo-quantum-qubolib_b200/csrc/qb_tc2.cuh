@@ -171,13 +171,18 @@ inline bool tc2_u16_eligible(int n, const double* W, float* dmin) {
 // kernel then works in units of 1/sigma, sigma a power of two applied to W: every MMA operand
 // (the y coupling rows, T(u), the column term's constant part, the gammas of the corrections)
 // is rounded to an integer in those units, so the accumulators are integers and the 16-bit
-// epilogue stays exact on the rounded values.  Per state the roundings add at most 4.5 units
-// (seven y rows, T and E_U at 0.5 each), the three low t bits' couplings 1.5, the partner's
-// gammas 2 (three chunk couplings and the sum of the others), plus fp32 rounding of the row
-// terms and of T below 2^-18 sum|Q| sigma; eps = 10 / sigma + 2^-16 sum|Q| bounds it (unscaled)
-// and pass 2 re-walks every record within 2 eps of the minimum in FP64.  Applies when, at the largest such sigma, every y coupling
-// row stays within +-2047 units, the value span with the chunk offsets and a 40-unit margin
-// within 2^16 units, and the span covers at least 1024 units.  W: the unscaled n x n FP64 W.
+// epilogue stays exact on the rounded values.  The column term takes half of what the roundings
+// of a column's seven y rows and three low t rows leave over before it is rounded itself, so that
+// a row, in the state or not, adds at most a quarter unit: 2.5 units per state and 0.5 of the
+// column term, for the partner 0.75 of the three chunk couplings of gamma, halved the same way,
+// and 0.5 of their sum with the others.  Measured against FP64 (rms in units, n = 20 .. 24, float
+// and wide integer Q): 0.55 for a pair's tile t and 0.66 for the partner; 0.86 and 0.96 with
+// every row's rounding left where it falls.  fp32 rounding of the row terms and of the column
+// term adds less than 2^-18 sum|Q| sigma.  eps = 10 / sigma + 2^-16 sum|Q| bounds it all
+// (unscaled), and pass 2 re-walks every record within 2 eps of the minimum in FP64.  Applies
+// when, at the largest such sigma, every y coupling row stays within +-2047 units, the value span
+// with the chunk offsets and a 40-unit margin within 2^16 units, and the span covers at least
+// 1024 units.  W: the unscaled n x n FP64 W.
 // On success: sigma, dmin (the lower bound of the rounded values in units, an integer) and eps.
 inline bool tc2_u16_quantized(int n, const double* W, double abs_sum, double* sigma, float* dmin, double* eps) {
   if (n < 20) return false;
@@ -224,6 +229,8 @@ inline void tc2_u16_tables(const float* gamma, float dmin, Tc2Tab* Q) {
   Q->dmin = dmin;
   int64_t g[8];
   for (int j = 0; j < 8; ++j) g[j] = (int64_t)std::llrint(gamma[j]);
+  double left = 0.0;  // half of what rounding the chunk couplings leaves over
+  for (int b : kTc2ChunkBits) left += 0.5 * ((double)gamma[b] - (double)g[b]);
   for (int b = 0; b < 3; ++b) Q->gx[b] = (float)g[kTc2ChunkBits[b]];
   for (int neg = 0; neg < 2; ++neg) {
     const int64_t s = neg ? -1 : 1;
@@ -240,7 +247,7 @@ inline void tc2_u16_tables(const float* gamma, float dmin, Tc2Tab* Q) {
         uint32_t h[2];
         for (int d = 0; d < 2; ++d) {
           // rounded as one sum: half a unit off at most, whatever the number of couplings
-          const double y = (d ? (double)gamma[0] : 0.0) + ((k & 1) ? (double)gamma[1] : 0.0) +
+          const double y = left + (d ? (double)gamma[0] : 0.0) + ((k & 1) ? (double)gamma[1] : 0.0) +
                            ((k & 2) ? (double)gamma[2] : 0.0) + ((k & 4) ? (double)gamma[3] : 0.0) +
                            (hh ? (double)gamma[7] : 0.0);
           const int64_t gp = (int64_t)std::llrint(y);
@@ -866,9 +873,11 @@ __global__ void __launch_bounds__(kTc2Threads, 1) tc_pair_kernel(const __grid_co
     // different ones.  (n = 20: the whole kernel 31 -> 18 thousand cycles.)
     const int kb0 = n - 17 - KW;  // variable of block bit 0 (block bit k: kb0 - k)
     if (warp < 8) {
-      // the column term's constant part E_U(u) + X(u) + 2^23 - Dlow, u = tid
+      // column u = tid: E_U(u), and the B operand's constant rows -- the couplings of the y
+      // variables (one exact fp16 integer each) and of the low t bits (two exact digits each);
+      // half of what the rows' rounding leaves over goes to E_U
       const int u = tid;
-      double e = 0.0;
+      double e = 0.0, left = 0.0;
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const double* row = Ws + (n - 1 - j) * n;
@@ -877,9 +886,26 @@ __global__ void __launch_bounds__(kTc2Threads, 1) tc_pair_kernel(const __grid_co
         for (int j2 = 0; j2 < j; ++j2) r += ((u >> j2) & 1) ? row[n - 1 - j2] : 0.0;
         e += ((u >> j) & 1) ? r : 0.0;
       }
-      const double x = ((u >> 4) & 1 ? (double)Tb.gx[0] : 0.0) + ((u >> 5) & 1 ? (double)Tb.gx[1] : 0.0) +
-                       ((u >> 6) & 1 ? (double)Tb.gx[2] : 0.0);
-      EU[u] = (float)(rint(e) + x + (double)Tb.k0s[0]);
+      unsigned char* Bu = Bsm + kmaj_off(u, 0);
+#pragma unroll
+      for (int i = 0; i < 10; ++i) {  // i < 7: y variable i; else low t bit i - 7
+        const double* row = Ws + (i < 7 ? n - 9 - i : n - 17 - (i - 7)) * n;
+        double v = 0.0;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v += ((u >> j) & 1) ? row[n - 1 - j] : 0.0;
+        const double w = rint(v);
+        left += v - w;
+        const float r = (float)w;
+        const float d1 = i < 7 ? 0.f : floorf(r * (1.0f / 2048.0f));
+        const __half h0 = __float2half_rn(fmaf(-2048.0f, d1, r)), h1 = __float2half_rn(d1);
+#pragma unroll
+        for (int s = 0; s < kTc2BStages; ++s) {
+          unsigned char* Bs = Bu + s * kTcN * 32;
+          *reinterpret_cast<__half*>(Bs + kmaj_off(0, i < 7 ? i : tc2_low_slot(i - 7, 0))) = h0;
+          if (i >= 7) *reinterpret_cast<__half*>(Bs + kmaj_off(0, tc2_low_slot(i - 7, 1))) = h1;
+        }
+      }
+      EU[u] = (float)(e + 0.5 * left);
     } else if (warp < 12) {
       // low t bits (pattern p = 2 st + b: bit 0 the pair's) x row couplings, y = tid - 256
       const int y = tid - 256;
@@ -947,30 +973,6 @@ __global__ void __launch_bounds__(kTc2Threads, 1) tc_pair_kernel(const __grid_co
           }
         }
         LO[p * kTc2LoCols + c] = v;
-      }
-    }
-    // B operand, constant columns: coupling rows of the y variables (one exact fp16 integer
-    // each) and of the low t bits (two exact digits each)
-    for (int e = tid; e < kTcN * 10; e += kTc2Threads) {
-      const int u = e & (kTcN - 1), i = e >> 8;  // i < 7: y variable i; else low t bit i - 7
-      const double* row = Ws + (i < 7 ? n - 9 - i : n - 17 - (i - 7)) * n;
-      double v = 0.0;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) v += ((u >> j) & 1) ? row[n - 1 - j] : 0.0;
-      const float r = (float)rint(v);
-      if (i < 7) {
-        const __half hv = __float2half_rn(r);
-#pragma unroll
-        for (int s = 0; s < kTc2BStages; ++s) *reinterpret_cast<__half*>(Bsm + s * kTcN * 32 + kmaj_off(u, i)) = hv;
-      } else {
-        const float d1 = floorf(r * (1.0f / 2048.0f));
-        const __half h0 = __float2half_rn(fmaf(-2048.0f, d1, r)), h1 = __float2half_rn(d1);
-        const int k0 = tc2_low_slot(i - 7, 0), k1 = tc2_low_slot(i - 7, 1);
-#pragma unroll
-        for (int s = 0; s < kTc2BStages; ++s) {
-          *reinterpret_cast<__half*>(Bsm + s * kTcN * 32 + kmaj_off(u, k0)) = h0;
-          *reinterpret_cast<__half*>(Bsm + s * kTcN * 32 + kmaj_off(u, k1)) = h1;
-        }
       }
     }
     fence_proxy_async();
@@ -1085,6 +1087,11 @@ __global__ void __launch_bounds__(kTc2Threads, 1) tc_pair_kernel(const __grid_co
       ok = !fail;
     } else if (warp == 2) {
       // ---------------------------------------------------------- B producer (once per block)
+      // X(u) + 2^23 - Dlow of the lane's columns u = lane + 32 r, by r & 3: u4 is lane bit 4
+      float xk[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        xk[c] = Tb.k0s[0] + ((lane >> 4) ? Tb.gx[0] : 0.f) + ((c & 1) ? Tb.gx[1] : 0.f) + ((c & 2) ? Tb.gx[2] : 0.f);
       for (uint32_t p = 0; p < nblk && ok; ++p) {
         const uint32_t jg = bbase + p;
         const uint32_t sa = jg & (uint32_t)(kTcParamSlots - 1), bs = jg & (uint32_t)(kTc2BStages - 1);
@@ -1106,8 +1113,8 @@ __global__ void __launch_bounds__(kTc2Threads, 1) tc_pair_kernel(const __grid_co
             if (r & 1) cr += f5;
             if (r & 2) cr += f6;
             if (r & 4) cr += f7;
-            // T(u) + the constant part: an integer in (0, 2^24), three exact digits
-            const float c = rintf(cr) + EU[lane + 32 * r];
+            // the whole column term: an integer in (0, 2^24), three exact digits
+            const float c = rintf(cr + EU[lane + 32 * r]) + xk[r & 3];
             const float d2 = floorf(c * (1.0f / 32768.0f)), rem = fmaf(-32768.0f, d2, c);
             const float d1 = floorf(rem * (1.0f / 2048.0f));
             dg[r] = __floats2half2_rn(fmaf(-2048.0f, d1, rem), d1);
