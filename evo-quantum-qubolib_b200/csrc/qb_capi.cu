@@ -650,6 +650,17 @@ int begin_finish_pass1(qb_handle* h, Plan& P, double* local_min) {
   return QB_OK;
 }
 
+// QB_F1's suffix step: row is the lexicographic minimum of best's prefix.  Exact arithmetic finds
+// best's energy again.  With float Q the two walks round differently and may pass over states
+// that tie to within rounding: then the lower energy stands.  False: integer Q disagrees.
+bool take_row(const Plan& P, const qb::ExactOut& row, qb::ExactOut* best) {
+  if (row.e > best->e) return !P.is_int;
+  if (row.e < best->e && P.is_int) return false;
+  best->x = row.x;
+  best->e = row.e;
+  return true;
+}
+
 // qb_solve of one whole problem: after pass 1 the minimum, the selection, the exact
 // re-evaluation and the final pick (with QB_F1's suffix step) follow on the device, then one copy
 // of the control block to the host.  The 16-bit pair kernel reduces its records' minimum itself,
@@ -721,10 +732,7 @@ int solve_fused(qb_handle* h, const Plan& P, qb_result* r) {
   const bool zero = !exact_form && P.is_int && P.eps == 0.0 && pass1_min >= 0.0;
   qb::ExactOut b = zero ? qb::ExactOut{0.0, 0ull, 0ull} : c.best;
   const bool found = zero || exact_form || c.count > 0;
-  if (found && P.rule.kind == qb::kTieQBF1 && b.x != 0) {
-    if (c.row.e != b.e) return QB_ECUDA;
-    b.x = c.row.x;
-  }
+  if (found && P.rule.kind == qb::kTieQBF1 && b.x != 0 && !take_row(P, c.row, &b)) return QB_ECUDA;
   memset(r, 0, sizeof(*r));
   r->form_used = P.form;
   r->is_integer = P.is_int ? 1 : 0;
@@ -808,23 +816,21 @@ bool lex_less_h(const qb::ExactOut& a, const qb::ExactOut& b) {
   return a.e < b.e || (a.e == b.e && a.key < b.key);
 }
 
-// QB_F1 rule, final step: smallest 18-bit suffix of the winning prefix with E == e_star.
-int qbf1_row(qb_handle* h, const Plan& P, uint64_t X, double e_star, uint64_t* Xout) {
+// QB_F1 rule, final step: smallest 18-bit suffix of the winning prefix with best's energy.
+int qbf1_row(qb_handle* h, const Plan& P, qb::ExactOut* best) {
   qb::RecGeom g{};
   g.kind = qb::kGeomBlock;
   g.n = P.n;
   g.fbits = 18;
   qb::TieRule nat{qb::kTieNatural, P.n, 0, 0, 0};
-  uint64_t rid = X >> 18;
+  uint64_t rid = best->x >> 18;
   QB_CUDA(h->cand.ensure(sizeof(uint64_t)));
   QB_CUDA(cudaMemcpyAsync(h->cand.p, &rid, sizeof(uint64_t), cudaMemcpyHostToDevice, h->st));
   h->h2d += (int64_t)sizeof(uint64_t);
   std::vector<qb::ExactOut> o;
   int rc = rescore(h, P, nat, g, 1, o);
   if (rc) return rc;
-  if (o.empty() || o[0].e != e_star) return QB_ECUDA;
-  *Xout = o[0].x;
-  return QB_OK;
+  return !o.empty() && take_row(P, o[0], best) ? QB_OK : QB_ECUDA;
 }
 
 }  // namespace
@@ -889,10 +895,8 @@ int qb_solve_finish(qb_handle* h, double global_min, qb_result* r) {
     r->candidate_records = count;
   }
   if (found && P.rule.kind == qb::kTieQBF1 && best.x != 0) {
-    uint64_t X;
-    int rc = qbf1_row(h, P, best.x, best.e, &X);
+    int rc = qbf1_row(h, P, &best);
     if (rc) return rc;
-    best.x = X;
   }
   QB_CUDA(cudaEventRecord(h->ev[3], h->st));
   QB_CUDA(cudaEventSynchronize(h->ev[3]));
