@@ -15,6 +15,7 @@
 #include "qb_common.cuh"
 #include "qb_exact.cuh"
 #include "qb_gray.cuh"
+#include "qb_host.cuh"
 #include "qb_qbf1.cuh"
 #include "qb_reduce.cuh"
 #include "qb_tc.cuh"
@@ -1451,15 +1452,31 @@ int batch_run(qb_handle* h, const qb_problem* problems, const std::vector<int32_
   if (graph) {
     // one graph launch per batch; the graph is captured again whenever the batch's shape, the
     // options or any buffer address differ from the captured one
-    std::vector<uint64_t> key = {(uint64_t)m, (uint64_t)w_total, (uint64_t)ar.size, (uint64_t)cap,
-                                 (uint64_t)gitems.size(), (uint64_t)uitems.size(), (uint64_t)gray_ids.size(),
-                                 (uint64_t)first.size(), (uint64_t)sm_gtab, (uint64_t)sm_gray, (uint64_t)sm_exact,
-                                 (uint64_t)sm_tc, (uint64_t)any_gray, (uint64_t)tc_pair, (uint64_t)(uintptr_t)Wall,
-                                 (uint64_t)(uintptr_t)h->hstage.p, (uint64_t)(uintptr_t)h->hout.p,
-                                 (uint64_t)(uintptr_t)h->own};
-    for (int k : {0, 1, 6, 7, 8}) key.push_back((uint64_t)(uintptr_t)B[k].p);
+    qb::BatchShape shape{};
+    shape.problems = (uint64_t)m;
+    shape.w_doubles = w_total;
+    shape.arena_bytes = ar.size;
+    shape.cap = (uint64_t)cap;
+    shape.gtab_items = gitems.size();
+    shape.units = uitems.size();
+    shape.selections = gray_ids.size();
+    shape.tc_runs = first.size();
+    shape.sm_gtab = sm_gtab;
+    shape.sm_gray = sm_gray;
+    shape.sm_exact = sm_exact;
+    shape.sm_tc = sm_tc;
+    shape.any_gray = any_gray;
+    shape.tc_pair = tc_pair;
+    shape.tc_n_max = (uint64_t)n_tc_max;
+    int i = 0;
     for (size_t off : {off_inst, off_git, off_uit, off_gid, off_item, off_first, off_tab, off_res, off_cand})
-      key.push_back((uint64_t)off);
+      shape.offsets[i++] = off;
+    i = 0;
+    for (const void* a : {(const void*)Wall, (const void*)h->hstage.p, (const void*)h->hout.p, (const void*)h->own,
+                          (const void*)B[0].p, (const void*)B[1].p, (const void*)B[6].p, (const void*)B[7].p,
+                          (const void*)B[8].p})
+      shape.addresses[i++] = (uint64_t)(uintptr_t)a;
+    const std::vector<uint64_t> key = qb::batch_graph_key(shape);
     if (!h->batch_graph || key != h->batch_graph_key) {
       if (h->batch_graph) {
         cudaGraphExecDestroy(h->batch_graph);

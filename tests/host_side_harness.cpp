@@ -1,0 +1,19 @@
+// Host-only harness for tests/test_host_side.py: exports the parts of the library's host side
+// that need no CUDA call.  Built by the test with g++; not part of the library.
+#include "qb_host.cuh"
+
+#include <cstring>
+
+extern "C" {
+
+// The graph key of a BatchShape given as its uint64 fields; returns the key's length.
+int h_batch_graph_key(const uint64_t* fields, int nfields, uint64_t* out, int room) {
+  qb::BatchShape s{};
+  if (nfields * 8 != (int)sizeof(s)) return -1;
+  memcpy(&s, fields, sizeof(s));
+  const std::vector<uint64_t> k = qb::batch_graph_key(s);
+  for (int i = 0; i < (int)k.size() && i < room; ++i) out[i] = k[i];
+  return (int)k.size();
+}
+
+}  // extern "C"

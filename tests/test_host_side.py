@@ -1,0 +1,76 @@
+"""Host side of the library that needs no GPU (csrc/qb_host.cuh), through a g++ harness."""
+import ctypes
+import os
+import shutil
+import subprocess
+
+import numpy as np
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+CSRC = os.path.join(os.path.dirname(HERE), "evo-quantum-qubolib_b200", "csrc")
+
+
+@pytest.fixture(scope="module")
+def harness(tmp_path_factory):
+    gxx = shutil.which("g++")
+    if gxx is None:
+        pytest.skip("g++ is not available")
+    out = str(tmp_path_factory.mktemp("host") / "host_side.so")
+    subprocess.run([gxx, "-std=c++17", "-O1", "-fPIC", "-shared", "-I", CSRC,
+                    os.path.join(HERE, "host_side_harness.cpp"), "-o", out], check=True)
+    return ctypes.CDLL(out)
+
+
+# --- the key under which a captured batch graph is replayed ------------------------------
+NAMES = ("problems", "w_doubles", "arena_bytes", "cap", "gtab_items", "units", "selections", "tc_runs", "sm_gtab",
+         "sm_gray", "sm_exact", "sm_tc", "any_gray", "tc_pair", "tc_n_max")
+FIELDS = len(NAMES) + 9 + 9
+
+
+def _key(harness, fields):
+    f = (ctypes.c_uint64 * FIELDS)(*fields)
+    out = (ctypes.c_uint64 * 64)()
+    k = harness.h_batch_graph_key(f, FIELDS, out, 64)
+    assert 0 < k <= 64
+    return list(out[:k])
+
+
+def test_every_field_is_in_the_key(harness):
+    base = list(range(1, FIELDS + 1))
+    for i in range(FIELDS):
+        other = list(base)
+        other[i] += 1000
+        assert _key(harness, other) != _key(harness, base)
+
+
+def _shape(sizes, gl, sms=148):
+    """The fields of a batch of integer problems that take the 16-bit pair kernel from 24
+    variables and the exact form below 20 (restated from qb_solve_batch's planning)."""
+    tc = [n for n in sizes if n >= 24]
+    total = sum(1 << (n - 15 - gl.get(n, 5)) for n in tc)
+    per = -(-total // min(sms, total))
+    items, runs, left = 0, 1, per
+    for n in tc:
+        groups, g = 1 << (n - 15 - gl.get(n, 5)), 0
+        while g < groups:
+            take = min(left, groups - g)
+            items, g, left = items + 1, g + take, left - take
+            if left == 0:
+                runs, left = runs + 1, per
+    runs += left != per
+    pre = sum(1 << (n - min(n, 16)) for n in sizes if n < 20)
+    smem = max((n * n + 1 + max(0, f - 13) * 288 + n * (n + 1) // 2) * 8
+               for n, f in [(n, gl.get(n, 5) + 12 if n >= 24 else min(n, 16)) for n in sizes])
+    return dict(problems=len(sizes), w_doubles=sum(n * n for n in sizes), arena_bytes=items, cap=pre + 4096,
+                selections=len(tc), tc_runs=runs, sm_exact=smem, tc_pair=1, tc_n_max=max(tc), sm_tc=121 * 1024)
+
+
+def test_batches_that_differ_in_the_largest_size_alone(harness):
+    """With wider records tuned for 26 variables, these two batches agree in everything but the
+    largest n, by which the search kernel lays out its shared memory: a replay of one's graph for
+    the other would write W over the barriers behind it."""
+    a, b = _shape([26, 32, 9], {26: 8}), _shape([26, 33, 4], {26: 8})
+    assert {k for k in a if a[k] != b[k]} == {"tc_n_max"}
+    keys = [_key(harness, [s.get(n, 0) for n in NAMES] + [0] * 18) for s in (a, b)]
+    assert keys[0] != keys[1]
