@@ -572,6 +572,7 @@ int begin_launch(qb_handle* h, const qb_problem* p, const qb_options* o, Plan& P
   if (rc) return rc;
   rc = plan_problem(h, o, P);
   if (rc) return rc;
+  if (fused && P.form == QB_FORM_EXACT && !qb::exact_form_fits(P.rec_count)) return QB_ENOMEM;
   if (P.form == QB_FORM_TC) {  // pair form: couplings of variable n-16 with the u variables
     for (int j = 0; j < 8; ++j) P.tc.gamma[j] = (float)(W[(size_t)(P.n - 16) * P.n + (P.n - 1 - j)] * P.tc.scale);
     const bool no16 = (o->flags & QB_FLAG_TC_NO16) != 0;

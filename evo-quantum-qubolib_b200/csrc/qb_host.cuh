@@ -5,6 +5,13 @@
 
 namespace qb {
 
+// The exact form's largest whole-problem search: 2^32 records of 2^16 states (n = 48).  Its
+// sharded form holds 24 bytes per record, 103 GB here, and refuses more for want of memory; the
+// whole-problem form holds next to nothing and would keep the GPU busy in one launch, for
+// minutes at n = 49 and for weeks at n = 62.
+constexpr uint64_t kExactMaxRecords = 1ull << 32;
+inline bool exact_form_fits(uint64_t records) { return records <= kExactMaxRecords; }
+
 // Everything a captured batch graph holds by value: copy sizes, grids, shared-memory sizes, the
 // kernels' scalar parameters and the buffers' addresses.  A batch may replay the graph of an
 // earlier one only where all of it is equal; the arrays the copies carry may differ.

@@ -16,4 +16,6 @@ int h_batch_graph_key(const uint64_t* fields, int nfields, uint64_t* out, int ro
   return (int)k.size();
 }
 
+int h_exact_form_fits(uint64_t records) { return qb::exact_form_fits(records) ? 1 : 0; }
+
 }  // extern "C"

@@ -74,3 +74,13 @@ def test_batches_that_differ_in_the_largest_size_alone(harness):
     assert {k for k in a if a[k] != b[k]} == {"tc_n_max"}
     keys = [_key(harness, [s.get(n, 0) for n in NAMES] + [0] * 18) for s in (a, b)]
     assert keys[0] != keys[1]
+
+
+# --- the exact form's limit ---------------------------------------------------------------
+@pytest.mark.parametrize("n", range(20, 63))
+def test_exact_form_limit(harness, n):
+    """Whole problems beyond the 2^32 records whose results (24 bytes each) a 180 GB GPU can hold
+    are refused, as they are when every record's result is kept."""
+    harness.h_exact_form_fits.argtypes = [ctypes.c_uint64]
+    records = 1 << (n - 16)
+    assert harness.h_exact_form_fits(records) == (records * 24 <= 180 << 30)
