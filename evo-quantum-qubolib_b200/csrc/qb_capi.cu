@@ -170,64 +170,12 @@ int cuda_fail(cudaError_t e) {
     if (_e != cudaSuccess) return cuda_fail(_e); \
   } while (0)
 
-int dtype_size(int dt) {
-  switch (dt) {
-    case QB_F32: return 4;
-    case QB_F64: return 8;
-    case QB_I8: return 1;
-    case QB_I16: return 2;
-    case QB_I32: return 4;
-    case QB_I64: return 8;
-    default: return 0;
-  }
-}
-
-template <class T>
-int host_problem_typed(const qb_problem* p, double* Wout, double* abs_sum) {
-  const int n = p->n;
-  const T* src = static_cast<const T*>(p->q);
-  const size_t ld = (size_t)p->ldq;
-  double s = 0.0;
-  bool bad = false;
-  for (int i = 0; i < n; ++i) {
-    const T* row = src + i * ld;
-    const double d = (double)row[i];
-    bad |= !std::isfinite(d);
-    s += std::fabs(d);
-    Wout[(size_t)i * n + i] = d;
-    for (int j = i + 1; j < n; ++j) {
-      const double a = (double)row[j], b = (double)src[j * ld + i];
-      bad |= !std::isfinite(a) || !std::isfinite(b);
-      s += std::fabs(a) + std::fabs(b);
-      Wout[(size_t)i * n + j] = Wout[(size_t)j * n + i] = a + b;
-    }
-  }
-  if (bad) return QB_EINVAL;
-  *abs_sum = s;
-  return QB_OK;
-}
-
-// Q in host memory (any dtype) -> W (n x n doubles, written to Wout) and sum |Q_ij|, without
-// intermediate copies (the batched search packs thousands of these).
-int load_host_problem_into(const qb_problem* p, double* Wout, double* abs_sum, bool* is_int) {
-  *is_int = p->dtype >= QB_I8;
-  switch (p->dtype) {
-    case QB_F32: return host_problem_typed<float>(p, Wout, abs_sum);
-    case QB_F64: return host_problem_typed<double>(p, Wout, abs_sum);
-    case QB_I8: return host_problem_typed<int8_t>(p, Wout, abs_sum);
-    case QB_I16: return host_problem_typed<int16_t>(p, Wout, abs_sum);
-    case QB_I32: return host_problem_typed<int32_t>(p, Wout, abs_sum);
-    case QB_I64: return host_problem_typed<int64_t>(p, Wout, abs_sum);
-    default: return QB_EINVAL;
-  }
-}
-
 // Q (any dtype, host or device) -> W (n x n doubles) and sum |Q_ij|.
 int load_problem(qb_handle* h, const qb_problem* p, std::vector<double>& W, double* abs_sum, bool* is_int) {
   const int n = p->n;
   W.resize((size_t)n * n);
-  if (!p->q_on_device) return load_host_problem_into(p, W.data(), abs_sum, is_int);
-  const int es = dtype_size(p->dtype);
+  if (!p->q_on_device) return qb::load_host_problem_into(p, W.data(), abs_sum, is_int);
+  const int es = qb::dtype_size(p->dtype);
   QB_CUDA(h->hraw.ensure((size_t)n * n * es));
   QB_CUDA(cudaMemcpy2DAsync(h->hraw.p, (size_t)n * es, p->q, (size_t)p->ldq * es, (size_t)n * es, n,
                             cudaMemcpyDeviceToHost, h->st));
@@ -237,7 +185,7 @@ int load_problem(qb_handle* h, const qb_problem* p, std::vector<double>& W, doub
   host.q = h->hraw.p;
   host.ldq = n;
   host.q_on_device = 0;
-  return load_host_problem_into(&host, W.data(), abs_sum, is_int);
+  return qb::load_host_problem_into(&host, W.data(), abs_sum, is_int);
 }
 
 int make_rule(const qb_options* o, int n, qb::TieRule* r) {
@@ -555,7 +503,7 @@ namespace {
 // validation, problem upload and the pass-1 launch of qb_solve_begin
 // (fused: qb_solve's whole-problem path, whose exact form has no pass 1)
 int begin_launch(qb_handle* h, const qb_problem* p, const qb_options* o, Plan& P, bool fused) {
-  if (p->n < 1 || p->n > qb::kMaxN || !p->q || p->ldq < p->n || dtype_size(p->dtype) == 0) return QB_EINVAL;
+  if (p->n < 1 || p->n > qb::kMaxN || !p->q || p->ldq < p->n || qb::dtype_size(p->dtype) == 0) return QB_EINVAL;
   if (o->shard_count > 1 && (o->shard_index < 0 || o->shard_index >= o->shard_count)) return QB_EINVAL;
   QB_CUDA(cudaSetDevice(h->device));
   h->st = o->stream ? static_cast<cudaStream_t>(o->stream) : h->own;
@@ -1202,7 +1150,7 @@ int batch_run(qb_handle* h, const qb_problem* problems, const std::vector<int32_
         const qb_problem* p = &problems[ids[j]];
         if (p->q_on_device) continue;
         bool ii = false;
-        rcs[j] = load_host_problem_into(p, Wall + w_offs[j], &sums[j], &ii);
+        rcs[j] = qb::load_host_problem_into(p, Wall + w_offs[j], &sums[j], &ii);
         ints[j] = ii;
         pair_fit(j);
       }
@@ -1588,7 +1536,7 @@ int qb_solve_batch(qb_handle* h, const qb_problem* problems, int32_t count, cons
   const bool form_ok = o->form == QB_FORM_AUTO || o->form == QB_FORM_GRAY;
   for (int32_t i = 0; i < count; ++i) {
     const qb_problem* p = &problems[i];
-    if (p->n < 1 || p->n > qb::kMaxN || !p->q || p->ldq < p->n || dtype_size(p->dtype) == 0) return QB_EINVAL;
+    if (p->n < 1 || p->n > qb::kMaxN || !p->q || p->ldq < p->n || qb::dtype_size(p->dtype) == 0) return QB_EINVAL;
     if (rule_ok && form_ok && o->shard_count <= 1 && p->n <= kBatchMaxN)
       batched.push_back(i);
     else
@@ -1611,7 +1559,7 @@ int qb_solve_batch(qb_handle* h, const qb_problem* problems, int32_t count, cons
 
 int qb_prefix_minima(qb_handle* h, const qb_problem* p, int32_t prefix_bits, double* out) {
   if (!h || !p || !out) return QB_EINVAL;
-  if (p->n < 1 || p->n > qb::kMaxN || !p->q || p->ldq < p->n || dtype_size(p->dtype) == 0) return QB_EINVAL;
+  if (p->n < 1 || p->n > qb::kMaxN || !p->q || p->ldq < p->n || qb::dtype_size(p->dtype) == 0) return QB_EINVAL;
   const int n = p->n;
   const int A = prefix_bits < 0 ? n - std::min(n, 20) : prefix_bits;
   const int B = n - A;
@@ -1668,7 +1616,7 @@ int qb_prefix_minima(qb_handle* h, const qb_problem* p, int32_t prefix_bits, dou
 }
 
 int qb_autotune(qb_handle* h, int32_t n, int32_t dtype, int32_t* form_out) {
-  if (!h || !form_out || n < 1 || n > qb::kMaxN || dtype_size(dtype) == 0) return QB_EINVAL;
+  if (!h || !form_out || n < 1 || n > qb::kMaxN || qb::dtype_size(dtype) == 0) return QB_EINVAL;
   const bool is_int = dtype >= QB_I8;
   qb_handle::Tuned& T = h->tuned[is_int ? 1 : 0][n];
   if (n < 20) {  // the exact form is the only one below 20 variables

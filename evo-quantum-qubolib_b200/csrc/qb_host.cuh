@@ -1,7 +1,12 @@
 // qb_host.cuh -- host-only parts of the library that need no CUDA call.
 #pragma once
+#include <cmath>
 #include <cstdint>
+#include <cstring>
 #include <vector>
+
+#include "../../include/qubo_b200.h"
+#include "qb_common.cuh"
 
 namespace qb {
 
@@ -33,6 +38,70 @@ inline std::vector<uint64_t> batch_graph_key(const BatchShape& s) {
   k.insert(k.end(), s.offsets, s.offsets + 9);
   k.insert(k.end(), s.addresses, s.addresses + 9);
   return k;
+}
+
+inline int dtype_size(int dt) {
+  switch (dt) {
+    case QB_F32: return 4;
+    case QB_F64: return 8;
+    case QB_I8: return 1;
+    case QB_I16: return 2;
+    case QB_I32: return 4;
+    case QB_I64: return 8;
+    default: return 0;
+  }
+}
+
+template <class T>
+int host_problem_typed(const qb_problem* p, double* Wout, double* abs_sum) {
+  const int n = p->n;
+  const T* src = static_cast<const T*>(p->q);
+  const size_t ld = (size_t)p->ldq;
+  double s = 0.0;
+  bool bad = false;
+  for (int i = 0; i < n; ++i) {
+    const T* row = src + i * ld;
+    const double d = (double)row[i];
+    bad |= !std::isfinite(d);
+    s += std::fabs(d);
+    Wout[(size_t)i * n + i] = d;
+    for (int j = i + 1; j < n; ++j) {
+      const double a = (double)row[j], b = (double)src[j * ld + i];
+      bad |= !std::isfinite(a) || !std::isfinite(b);
+      s += std::fabs(a) + std::fabs(b);
+      Wout[(size_t)i * n + j] = Wout[(size_t)j * n + i] = a + b;
+    }
+  }
+  if (bad) return QB_EINVAL;
+  *abs_sum = s;
+  return QB_OK;
+}
+
+// Q in host memory (any dtype, 1 <= n <= 62) -> W (n x n doubles, written to Wout) and sum |Q_ij|,
+// without intermediate copies (the batched search packs thousands of these) unless the address is
+// not a multiple of the element size, as a view into a byte buffer can have it.
+inline int load_host_problem_into(const qb_problem* p, double* Wout, double* abs_sum, bool* is_int) {
+  *is_int = p->dtype >= QB_I8;
+  const size_t es = (size_t)dtype_size(p->dtype);
+  if (es && (uintptr_t)p->q % es) {
+    alignas(8) unsigned char tmp[kMaxN * kMaxN * 8];
+    const size_t row = (size_t)p->n * es;
+    for (int i = 0; i < p->n; ++i)
+      memcpy(tmp + i * row, static_cast<const unsigned char*>(p->q) + (size_t)i * (size_t)p->ldq * es, row);
+    qb_problem at = *p;
+    at.q = tmp;
+    at.ldq = p->n;
+    return load_host_problem_into(&at, Wout, abs_sum, is_int);
+  }
+  switch (p->dtype) {
+    case QB_F32: return host_problem_typed<float>(p, Wout, abs_sum);
+    case QB_F64: return host_problem_typed<double>(p, Wout, abs_sum);
+    case QB_I8: return host_problem_typed<int8_t>(p, Wout, abs_sum);
+    case QB_I16: return host_problem_typed<int16_t>(p, Wout, abs_sum);
+    case QB_I32: return host_problem_typed<int32_t>(p, Wout, abs_sum);
+    case QB_I64: return host_problem_typed<int64_t>(p, Wout, abs_sum);
+    default: return QB_EINVAL;
+  }
 }
 
 }  // namespace qb

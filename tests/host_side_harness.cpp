@@ -18,4 +18,13 @@ int h_batch_graph_key(const uint64_t* fields, int nfields, uint64_t* out, int ro
 
 int h_exact_form_fits(uint64_t records) { return qb::exact_form_fits(records) ? 1 : 0; }
 
+// W and sum |Q| of a host matrix; sum and the integer flag in out[0], out[1]
+int h_load(const void* q, int n, int64_t ldq, int dtype, double* W, double* out) {
+  const qb_problem p{n, dtype, q, ldq, 0, 0};
+  bool is_int = false;
+  const int rc = qb::load_host_problem_into(&p, W, &out[0], &is_int);
+  out[1] = is_int;
+  return rc;
+}
+
 }  // extern "C"

@@ -3,22 +3,25 @@ import ctypes
 import os
 import shutil
 import subprocess
+import sys
 
-import numpy as np
 import pytest
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(os.path.dirname(HERE), "evo-quantum-qubolib_b200", "csrc")
+CUDA_INC = "/usr/local/cuda/include"
 
 
 @pytest.fixture(scope="module")
 def harness(tmp_path_factory):
     gxx = shutil.which("g++")
-    if gxx is None:
-        pytest.skip("g++ is not available")
+    if gxx is None or not os.path.isdir(CUDA_INC):
+        pytest.skip("g++ or the CUDA headers are not available")
     out = str(tmp_path_factory.mktemp("host") / "host_side.so")
-    subprocess.run([gxx, "-std=c++17", "-O1", "-fPIC", "-shared", "-I", CSRC,
-                    os.path.join(HERE, "host_side_harness.cpp"), "-o", out], check=True)
+    # a load from an address that its type does not allow stops the process
+    subprocess.run([gxx, "-std=c++17", "-O1", "-fPIC", "-shared", "-fsanitize=alignment",
+                    "-fsanitize-undefined-trap-on-error", "-I", CSRC,
+                    "-I", CUDA_INC, os.path.join(HERE, "host_side_harness.cpp"), "-o", out], check=True)
     return ctypes.CDLL(out)
 
 
@@ -84,3 +87,35 @@ def test_exact_form_limit(harness, n):
     harness.h_exact_form_fits.argtypes = [ctypes.c_uint64]
     records = 1 << (n - 16)
     assert harness.h_exact_form_fits(records) == (records * 24 <= 180 << 30)
+
+
+# --- matrices in host memory ----------------------------------------------------------------
+LOAD = """
+import ctypes, sys
+import numpy as np
+L = ctypes.CDLL(sys.argv[1])
+L.h_load.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_int64, ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p]
+n, ld, off, dt = int(sys.argv[2]), int(sys.argv[3]), int(sys.argv[4]), np.dtype(sys.argv[5])
+code = 1 + ["f4", "f8", "i1", "i2", "i4", "i8"].index(sys.argv[5])
+rng = np.random.default_rng(n)
+raw = np.zeros(n * ld * dt.itemsize + 16, np.uint8)
+raw = raw[(-raw.ctypes.data) % 8:]  # 8-byte aligned start
+Q = raw[off:off + n * ld * dt.itemsize].view(dt).reshape(n, ld)
+Q[:] = rng.integers(-50, 50, (n, ld)) if dt.kind == "i" else rng.standard_normal((n, ld))
+W, out = np.zeros((n, n)), np.zeros(2)
+assert L.h_load(Q.ctypes.data, n, ld, code, W.ctypes.data, out.ctypes.data) == 0
+D = Q[:, :n].astype(np.float64)
+want = D + D.T
+want[np.arange(n), np.arange(n)] = np.diag(D)
+assert np.array_equal(W, want) and abs(out[0] - np.abs(D).sum()) <= 1e-12 * out[0] and out[1] == (dt.kind == "i")
+"""
+
+
+# the offset in bytes from an aligned address; a leading dimension of n and beyond
+@pytest.mark.parametrize("dt,off", [("f4", 0), ("f4", 2), ("f8", 0), ("f8", 4), ("f8", 1), ("i1", 1), ("i2", 1), ("i4", 3),
+                                    ("i8", 4)])
+@pytest.mark.parametrize("n,ld", [(1, 1), (7, 9), (62, 62), (62, 65)])
+def test_host_matrix_at_any_address(harness, dt, off, n, ld):
+    p = subprocess.run([sys.executable, "-c", LOAD, harness._name, str(n), str(ld), str(off), dt], capture_output=True,
+                       text=True)
+    assert p.returncode == 0, p.stderr
