@@ -31,44 +31,32 @@
 
 namespace {
 
-struct DevBuf {
-  void* p = nullptr;
-  size_t cap = 0;
-  cudaError_t ensure(size_t bytes) {
-    if (bytes <= cap) return cudaSuccess;
-    if (p) cudaFree(p);
-    p = nullptr;
-    cap = 0;
-    const size_t want = std::max<size_t>(bytes + bytes / 8, 256);  // room for the next batch, a little larger
-    cudaError_t e = cudaMalloc(&p, want);
-    if (e == cudaSuccess) cap = want;
+struct DevAlloc {
+  static constexpr size_t kMin = 256;
+  static int alloc(void** p, size_t bytes) {
+    const cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaSuccess) cudaGetLastError();  // a later launch check must not see it
     return e;
   }
-  void release() {
-    if (p) cudaFree(p);
-    p = nullptr;
-    cap = 0;
-  }
+  static void release(void* p) { cudaFree(p); }
 };
 
-struct HostBuf {
-  void* p = nullptr;
-  size_t cap = 0;
-  cudaError_t ensure(size_t bytes) {
-    if (bytes <= cap) return cudaSuccess;
-    if (p) cudaFreeHost(p);
-    p = nullptr;
-    cap = 0;
-    const size_t want = std::max<size_t>(bytes + bytes / 8, 4096);
-    cudaError_t e = cudaMallocHost(&p, want);
-    if (e == cudaSuccess) cap = want;
+struct PinnedAlloc {
+  static constexpr size_t kMin = 4096;
+  static int alloc(void** p, size_t bytes) {
+    const cudaError_t e = cudaMallocHost(p, bytes);
+    if (e != cudaSuccess) cudaGetLastError();
     return e;
   }
-  void release() {
-    if (p) cudaFreeHost(p);
-    p = nullptr;
-    cap = 0;
-  }
+  static void release(void* p) { cudaFreeHost(p); }
+};
+
+struct DevBuf : qb::GrowBuf<DevAlloc> {
+  cudaError_t ensure(size_t bytes) { return (cudaError_t)GrowBuf::ensure(bytes); }
+};
+
+struct HostBuf : qb::GrowBuf<PinnedAlloc> {
+  cudaError_t ensure(size_t bytes) { return (cudaError_t)GrowBuf::ensure(bytes); }
 };
 
 constexpr double kTwo24 = 16777216.0;

@@ -1,5 +1,6 @@
 // qb_host.cuh -- host-only parts of the library that need no CUDA call.
 #pragma once
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
@@ -9,6 +10,34 @@
 #include "qb_common.cuh"
 
 namespace qb {
+
+// A buffer that grows on demand and keeps its room.  It takes an eighth more than asked, so that
+// the next, slightly larger call does not allocate again, but at most 16 MB more, and where that
+// much cannot be had just what is asked.  A: alloc(&p, bytes) (0 on success), release(p), kMin.
+template <class A>
+struct GrowBuf {
+  static constexpr size_t kMaxSlack = (size_t)16 << 20;
+  void* p = nullptr;
+  size_t cap = 0;
+  int ensure(size_t bytes) {
+    if (bytes <= cap) return 0;
+    release();
+    const size_t least = std::max(bytes, A::kMin), want = std::max(bytes + std::min(bytes / 8, kMaxSlack), A::kMin);
+    size_t got = want;
+    int e = A::alloc(&p, want);
+    if (e && want > least) e = A::alloc(&p, got = least);
+    if (e)
+      p = nullptr;
+    else
+      cap = got;
+    return e;
+  }
+  void release() {
+    if (p) A::release(p);
+    p = nullptr;
+    cap = 0;
+  }
+};
 
 // The exact form's largest whole-problem search: 2^32 records of 2^16 states (n = 48).  Its
 // sharded form holds 24 bytes per record, 103 GB here, and refuses more for want of memory; the

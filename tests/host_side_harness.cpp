@@ -4,7 +4,30 @@
 
 #include <cstring>
 
+namespace {
+size_t g_room, g_used;
+struct FakeAlloc {  // allocates from g_room bytes
+  static constexpr size_t kMin = 256;
+  static int alloc(void** p, size_t bytes) {
+    if (bytes > g_room) return 2;
+    g_used = bytes;
+    *p = &g_used;
+    return 0;
+  }
+  static void release(void*) { g_used = 0; }
+};
+}  // namespace
+
 extern "C" {
+
+// Grows one buffer to each size in turn with `room` bytes to be had: the bytes then in use, or 0
+// where the buffer refuses.
+void h_grow(uint64_t room, const uint64_t* sizes, int count, uint64_t* used) {
+  qb::GrowBuf<FakeAlloc> b;
+  g_room = room;
+  g_used = 0;
+  for (int i = 0; i < count; ++i) used[i] = b.ensure(sizes[i]) ? 0 : g_used;
+}
 
 // The graph key of a BatchShape given as its uint64 fields; returns the key's length.
 int h_batch_graph_key(const uint64_t* fields, int nfields, uint64_t* out, int room) {

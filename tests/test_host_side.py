@@ -119,3 +119,20 @@ def test_host_matrix_at_any_address(harness, dt, off, n, ld):
     p = subprocess.run([sys.executable, "-c", LOAD, harness._name, str(n), str(ld), str(off), dt], capture_output=True,
                        text=True)
     assert p.returncode == 0, p.stderr
+
+
+# --- buffers that grow on demand --------------------------------------------------------------
+def _grow(harness, room, sizes):
+    a, used = (ctypes.c_uint64 * len(sizes))(*sizes), (ctypes.c_uint64 * len(sizes))()
+    harness.h_grow(ctypes.c_uint64(room), a, len(sizes), used)
+    return list(used)
+
+
+def test_buffers_grow_by_little(harness):
+    big = 150 << 30
+    assert _grow(harness, 1 << 40, [1, 4000, 4500, 5000]) == [256, 4500, 4500, 5625]
+    assert all(u <= s + (16 << 20) for s, u in zip([1 << 30, big], _grow(harness, 1 << 40, [1 << 30, big])))
+    # what fits is not refused for the sake of spare room
+    assert _grow(harness, big, [big]) == [big]
+    assert _grow(harness, 1000, [1000, 999]) == [1000, 1000]
+    assert _grow(harness, 1000, [1001, 900]) == [0, 900]
