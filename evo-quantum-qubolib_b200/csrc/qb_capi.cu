@@ -304,6 +304,8 @@ void fill_plan_fields(const qb_handle* h, const Plan& P, qb_result* r) {
 
 constexpr size_t kCtlBytes = 128;  // SolveCtl's room before W
 static_assert(sizeof(qb::SolveCtl) <= kCtlBytes, "control block");
+constexpr size_t kAnswerBytes = 128;  // hmisc: an answer copied back
+static_assert(sizeof(qb::SolveCtl) <= kAnswerBytes && sizeof(qb::Qbf1Answer) <= kAnswerBytes, "room for the answer");
 
 qb::SolveCtl* dev_ctl(qb_handle* h) { return static_cast<qb::SolveCtl*>(h->W.p); }
 const double* dev_W(qb_handle* h) { return reinterpret_cast<const double*>(static_cast<char*>(h->W.p) + kCtlBytes); }
@@ -537,7 +539,7 @@ int begin_launch(qb_handle* h, const qb_problem* p, const qb_options* o, Plan& P
   rc = upload_W(h, W);
   if (rc) return rc;
   QB_CUDA(h->misc.ensure(64));
-  QB_CUDA(h->hmisc.ensure(64));
+  QB_CUDA(h->hmisc.ensure(kAnswerBytes));
   if (fused && P.form == QB_FORM_EXACT) return QB_OK;
   QB_CUDA(cudaEventRecord(h->ev[0], h->st));
   return run_pass1(h, P);
@@ -919,7 +921,6 @@ int qbf1_wrap_solve(qb_handle* h, const qb_problem* p, const qb_options* o, qb_r
   h->kernels += 4;
   QB_CUDA(cudaGetLastError());
   QB_CUDA(cudaEventRecord(h->ev[1], h->st));
-  static_assert(sizeof(qb::Qbf1Answer) <= 64, "hmisc");
   QB_CUDA(cudaMemcpyAsync(h->hmisc.p, ans, sizeof(qb::Qbf1Answer), cudaMemcpyDeviceToHost, h->st));
   h->d2h += (int64_t)sizeof(qb::Qbf1Answer);
   QB_CUDA(cudaStreamSynchronize(h->st));
@@ -965,7 +966,7 @@ int qb_solve(qb_handle* h, const qb_problem* p, const qb_options* o, qb_result* 
   if (!r) return QB_EINVAL;
   if (h && p && o && (o->flags & QB_FLAG_INT16_WRAP)) {
     if (o->tie_rule != QB_TIE_QB_F1) return QB_EINVAL;
-    QB_CUDA(h->hmisc.ensure(64));
+    QB_CUDA(h->hmisc.ensure(kAnswerBytes));
     const int rc = qbf1_wrap_solve(h, p, o, r);
     if (rc) r->status = rc;
     return rc;
