@@ -321,19 +321,23 @@ __device__ __forceinline__ bool mbar_wait_idle(uint64_t* b, uint32_t parity, vol
   }
 }
 
-// bounded wait of the epilogue and the MMA issue, as one statement without a result: a failed
-// wait (the limit ran out, or another role gave up) sets fail, which the caller looks at once
-// per block; with fail set, later waits return after one poll.  The usual path is one try_wait
-// and one branch.  The polls carry a 100 ns suspend hint (1.73 -> 1.72 ms per 2^36 states
-// against the default; 1 us on the first try as well 1.78 ms).
+// bounded wait of the epilogue and the MMA issue, by a converged warp, as one statement without a
+// result: a failed wait (the limit ran out, or another role gave up) sets fail, which the caller
+// looks at once per block; with fail set, later waits return after one poll.  Every branch is on
+// a vote, so that the warp stays together and fail is the same in all its lanes whatever the
+// lanes' polls and clocks say.  The usual path is one try_wait, one vote and one branch.  The
+// polls carry a 100 ns suspend hint (1.73 -> 1.72 ms per 2^36 states against the default; 1 us on
+// the first try as well 1.78 ms).
 __device__ __forceinline__ void mbar_wait_flag(uint32_t bar, uint32_t parity, uint32_t abort_addr, uint32_t& fail) {
   asm volatile(
       "{\n .reg .pred p, q;\n .reg .u64 t0, t1;\n .reg .u32 a;\n"
-      " mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n @p bra.uni DONE;\n"
-      " setp.ne.u32 q, %0, 0;\n @q bra.uni DONE;\n mov.u64 t0, %%globaltimer;\n"
-      "POLL:\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 100;\n @p bra.uni DONE;\n"
+      " mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n vote.sync.all.pred p, p, 0xffffffff;\n @p bra.uni DONE;\n"
+      " setp.ne.u32 q, %0, 0;\n vote.sync.any.pred q, q, 0xffffffff;\n @q bra.uni DONE;\n mov.u64 t0, %%globaltimer;\n"
+      "POLL:\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 100;\n vote.sync.all.pred p, p, 0xffffffff;\n"
+      " @p bra.uni DONE;\n"
       " ld.volatile.shared.u32 a, [%3];\n mov.u64 t1, %%globaltimer;\n sub.u64 t1, t1, t0;\n"
-      " setp.gt.u64 q, t1, %4;\n setp.ne.or.u32 q, a, 0, q;\n @!q bra.uni POLL;\n mov.u32 %0, 1;\n"
+      " setp.gt.u64 q, t1, %4;\n setp.ne.or.u32 q, a, 0, q;\n vote.sync.any.pred q, q, 0xffffffff;\n @!q bra.uni POLL;\n"
+      " mov.u32 %0, 1;\n"
       "DONE:\n}\n"
       : "+r"(fail)
       : "r"(bar), "r"(parity), "r"(abort_addr), "n"(kTcWaitLimitNs)
@@ -1095,7 +1099,8 @@ __global__ void __launch_bounds__(kTc2Threads, 1) tc_pair_kernel(const __grid_co
       for (uint32_t p = 0; p < nblk && ok; ++p) {
         const uint32_t jg = bbase + p;
         const uint32_t sa = jg & (uint32_t)(kTcParamSlots - 1), bs = jg & (uint32_t)(kTc2BStages - 1);
-        ok = mbar_wait_idle(&p_full[sa], (jg / kTcParamSlots) & 1u, abort_flag);
+        // the lanes' waits end apart, at the limit with different results: all go on or none does
+        ok = __all_sync(0xffffffffu, mbar_wait_idle(&p_full[sa], (jg / kTcParamSlots) & 1u, abort_flag));
         if (!ok) break;
         const Tc2Slot& sl = slots[sa];
         __half2 dg[8];
@@ -1137,7 +1142,7 @@ __global__ void __launch_bounds__(kTc2Threads, 1) tc_pair_kernel(const __grid_co
           for (int m = 0; m <= KW; ++m)
             if ((lp >> m) & 1) el += sl.c[m];
         }
-        ok = mbar_wait_idle(&b_empty[bs], ((jg / kTc2BStages) & 1u) ^ 1u, abort_flag);
+        ok = __all_sync(0xffffffffu, mbar_wait_idle(&b_empty[bs], ((jg / kTc2BStages) & 1u) ^ 1u, abort_flag));
         if (!ok) break;
         unsigned char* Bst = Bsm + bs * kTcN * 32;
 #pragma unroll
