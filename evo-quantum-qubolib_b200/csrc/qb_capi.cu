@@ -1574,6 +1574,20 @@ int qb_prefix_minima(qb_handle* h, const qb_problem* p, int32_t prefix_bits, dou
   qb::TieRule rule{qb::kTieNatural, n, 0, 0, 0};
   const qb::ProblemDev pd{n, dev_W(h)};
   const uint64_t count = 1ull << A;
+  if (B <= qb::kPrefixFewBits) {
+    QB_CUDA(h->exout.ensure(count * sizeof(double)));
+    QB_CUDA(h->hout.ensure(count * sizeof(double)));
+    const uint64_t ctas = std::min<uint64_t>(((1ull << n) + 255) >> 8, (uint64_t)h->sm_count * 8);
+    qb::prefix_few_states_kernel<<<(unsigned)ctas, qb::kExactThreads, (size_t)n * n * sizeof(double), h->st>>>(
+        pd, B, static_cast<double*>(h->exout.p));
+    ++h->kernels;
+    QB_CUDA(cudaGetLastError());
+    QB_CUDA(cudaMemcpyAsync(h->hout.p, h->exout.p, count * sizeof(double), cudaMemcpyDeviceToHost, h->st));
+    QB_CUDA(cudaStreamSynchronize(h->st));
+    const double* e = static_cast<const double*>(h->hout.p);
+    for (uint64_t i = 0; i < count; ++i) out[i] = e[qb::gray64(i)];  // QBF's prefix visiting order
+    return QB_OK;
+  }
   // few prefixes: each split over 2^sb CTAs (of at least 2^14 states) as long as all of them run
   // at once, two per SM; more CTAs repeat the set-up, fewer leave SMs idle.  Measured for the
   // whole call (us, the winner's thread walking again) at sb = 0 1 2 3 4 5: n = 27, A = 7 182 128 132 149 167 221; n = 24, A = 4

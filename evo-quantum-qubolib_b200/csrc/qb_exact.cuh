@@ -509,6 +509,41 @@ exact_records_kernel(ProblemDev P, TieRule R, RecGeom G, const uint64_t* __restr
   exact_record_body(P, R, G, rid, out + ((slot << split_bits) | part), smem_d, part, split_bits);
 }
 
+// qb_prefix_minima for prefixes of few states: out[p] = the minimum over the 2^B states of prefix p
+// (natural order), every energy summed from scratch, a state per thread and W loaded once per CTA.
+// In exact_records_kernel a prefix costs a CTA's whole set-up, which pays from 2^8 states on.  The
+// whole call (f64, us) there and here: n = 20, B = 0 .. 7 25254 12658 6386 3196 1649 848 448 238 and
+// 847 469 298 208 156 134 125 118; n = 22, B = 7 892 and 435; B = 8 there 470.
+constexpr int kPrefixFewBits = 7;
+__global__ void __launch_bounds__(kExactThreads)
+prefix_few_states_kernel(ProblemDev P, int B, double* __restrict__ out) {
+  extern __shared__ __align__(16) double smem_d[];
+  __shared__ double red[kExactThreads / 32];
+  const int n = P.n;
+  for (int i = threadIdx.x; i < n * n; i += kExactThreads) smem_d[i] = P.W[i];
+  __syncthreads();
+  const double inf = __longlong_as_double(0x7ff0000000000000ll);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lb = min(B, 5), g = 1 << (B - lb);  // a prefix: 2^lb lanes of g neighbouring warps
+  const uint64_t states = 1ull << n;
+  for (uint64_t x0 = (uint64_t)blockIdx.x * kExactThreads; x0 < states; x0 += (uint64_t)gridDim.x * kExactThreads) {
+    const uint64_t X = x0 + threadIdx.x;
+    double m = X < states ? energy_from_scratch(smem_d, n, X) : inf;
+    __syncwarp();
+    for (int b = 0; b < lb; ++b) {
+      const double o = __shfl_xor_sync(0xffffffffu, m, 1 << b);
+      m = o < m ? o : m;
+    }
+    if (g > 1) {
+      if (lane == 0) red[warp] = m;
+      __syncthreads();
+      for (int w = warp; w < warp + g && w < kExactThreads / 32; ++w) m = red[w] < m ? red[w] : m;
+      __syncthreads();
+    }
+    if (X < states && (X & mask64(B)) == 0) out[X >> B] = m;
+  }
+}
+
 // One solve's control words on the device, uploaded with W and copied back with the answer.
 struct SolveCtl {
   uint32_t err;      // error word of the tensor-core kernels
