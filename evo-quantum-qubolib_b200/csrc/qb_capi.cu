@@ -637,8 +637,8 @@ int solve_fused(qb_handle* h, const Plan& P, qb_result* r) {
   }
   if (maxf > qb::kExactMaxFree) return QB_EINVAL;
   const unsigned ctas = 2u * (unsigned)h->sm_count;
-  // parts of 2^13 states (no walked bits): at most 16 per candidate record, of which there are
-  // few; in the exact form as long as all CTAs run at once
+  // parts of 2^13 states (no walked bits): at most 16 per candidate record (fewer where there are
+  // many, which the kernel sees); in the exact form as long as all CTAs run at once
   int sb = std::max(0, std::min(4, maxf - 13));
   if (exact_form)
     while (sb > 0 && (P.rec_count << sb) > ctas) --sb;
