@@ -150,6 +150,7 @@ __device__ __forceinline__ ExactOut exact_record_min(const ProblemDev& P, const 
   __shared__ int var[kExactMaxFree];            // variables of the free bits, lowest bit first
   __shared__ double hs[64];                     // fields from the base state: sum of W_vq over its bits q != v
   __shared__ double q5[32];                     // energy of a register pattern alone
+  __shared__ uint64_t xg[32];                   // its state bits
   __shared__ double qo[1 << kExactLowWalk];     // energy of a pattern of the low walked bits alone
   __shared__ double Wt[8][8];                   // couplings of the thread bits, W_vv + field on the diagonal
   __shared__ double ct[2][16];                  // energy of a pattern of thread bits 0-3, 4-7 from the base state
@@ -230,9 +231,11 @@ __device__ __forceinline__ ExactOut exact_record_min(const ProblemDev& P, const 
     if (lane == 0) e_base = e + 0.5 * h;
   } else if (warp == 1) {
     double s = 0.0;  // register pattern g = lane
+    uint64_t xs = 0;
 #pragma unroll
     for (int u = 0; u < kExactRegBits; ++u) {
       if (u >= Lr) break;
+      xs |= ((uint64_t)(lane >> u) & 1ull) << (n - 1 - var[u]);
       const double* row = Ws + var[u] * n;
       double r = row[var[u]];
 #pragma unroll
@@ -240,6 +243,7 @@ __device__ __forceinline__ ExactOut exact_record_min(const ProblemDev& P, const 
       s += ((lane >> u) & 1) ? r : 0.0;
     }
     q5[lane] = s;
+    xg[lane] = xs;
   } else if (warp == 2) {
     const int half = lane >> 4, g = lane & 15;  // thread pattern g of bits 4 half ..
     double s = 0.0;
@@ -372,7 +376,12 @@ __device__ __forceinline__ ExactOut exact_record_min(const ProblemDev& P, const 
   for (int pass = 0; pass < 2; ++pass) {
     if (cand) {
       if (pass == 0 || steps > 1) start();  // without walked bits el still holds the start
-      uint64_t Xh = 0;
+      uint64_t Xh = 0;  // pass 1: the state's bits but for the register pattern's
+      if (pass == 1) {
+        Xh = base;
+        for (int j = 0; j < tb; ++j)
+          if ((t >> j) & 1) Xh |= 1ull << (n - 1 - var[L + j]);
+      }
       uint32_t st = 0;
       double target = best_e;
       const bool seek = pass == 1 && best_cnt == 1;
@@ -407,15 +416,9 @@ __device__ __forceinline__ ExactOut exact_record_min(const ProblemDev& P, const 
           uint32_t hit = 0;
 #pragma unroll
           for (int g = 0; g < 32; ++g) hit |= c + el[g] == target ? 1u << g : 0u;
-          uint64_t Xt = base | Xh;
-          for (int j = 0; j < tb; ++j)
-            if ((t >> j) & 1) Xt |= 1ull << (n - 1 - var[L + j]);
 #pragma unroll 1
           for (; hit; hit &= hit - 1) {
-            const int g = __ffs(hit) - 1;
-            uint64_t X = Xt;
-            for (int u = 0; u < Lr; ++u)
-              if ((g >> u) & 1) X |= 1ull << (n - 1 - var[u]);
+            const uint64_t X = Xh | xg[__ffs(hit) - 1];
             const uint64_t k = tie_key(R, X);
             if (k < best_k) {
               best_k = k;
