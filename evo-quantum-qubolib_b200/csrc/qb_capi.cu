@@ -110,8 +110,8 @@ struct qb_handle_s {
   cudaStream_t st = nullptr;
   DevBuf W;  // SolveCtl, then W (n*n doubles)
   DevBuf gtab, rec, cand, misc, exout;
-  DevBuf bat[15];  // qb_solve_batch: 0 W, 1 the small arrays and candidates, 6 outputs, 7 G tables, 8 records;
-                   // QB_F1's int16 form: 0 Q, 6 BB, 7 ABBA, 8 AA, 9 keys and answer
+  DevBuf bat[6];  // qb_solve_batch: 0 W, 1 the small arrays and candidates, 2 outputs, 3 G tables, 4 records;
+                  // QB_F1's int16 form: 0 Q, 2 BB, 3 ABBA, 4 AA, 5 keys and answer
   HostBuf hW, hmisc, hout, hbat;  // hW: the upload of W; hbat: qb_solve_batch's packed W matrices (pinned)
   HostBuf hraw;                    // a device matrix copied back (pinned)
   HostBuf hstage;                  // qb_solve_batch: descriptors and work lists (pinned)
@@ -890,18 +890,18 @@ int qbf1_wrap_solve(qb_handle* h, const qb_problem* p, const qb_options* o, qb_r
   const size_t cols = (size_t)1 << qb::kQbf1B;
   DevBuf* B = h->bat;
   QB_CUDA(B[0].ensure(Qi.size() * sizeof(int)));
-  QB_CUDA(B[6].ensure(cols * sizeof(short)));
-  QB_CUDA(B[7].ensure((size_t)A * cols * sizeof(short)));
-  QB_CUDA(B[8].ensure(steps * sizeof(uint32_t)));
+  QB_CUDA(B[2].ensure(cols * sizeof(short)));
+  QB_CUDA(B[3].ensure((size_t)A * cols * sizeof(short)));
+  QB_CUDA(B[4].ensure(steps * sizeof(uint32_t)));
   constexpr size_t key_bytes = qb::kQbf1Threads * sizeof(unsigned long long);
-  QB_CUDA(B[9].ensure(key_bytes + sizeof(qb::Qbf1Answer)));
+  QB_CUDA(B[5].ensure(key_bytes + sizeof(qb::Qbf1Answer)));
   QB_CUDA(cudaMemcpyAsync(B[0].p, Qi.data(), Qi.size() * sizeof(int), cudaMemcpyHostToDevice, h->st));
   h->h2d += (int64_t)(Qi.size() * sizeof(int));
   const int* dQ = static_cast<const int*>(B[0].p);
-  short* BB = static_cast<short*>(B[6].p);
-  short* ABBA = static_cast<short*>(B[7].p);
-  uint32_t* AA = static_cast<uint32_t*>(B[8].p);
-  unsigned long long* key = static_cast<unsigned long long*>(B[9].p);
+  short* BB = static_cast<short*>(B[2].p);
+  short* ABBA = static_cast<short*>(B[3].p);
+  uint32_t* AA = static_cast<uint32_t*>(B[4].p);
+  unsigned long long* key = static_cast<unsigned long long*>(B[5].p);
   qb::Qbf1Answer* ans = reinterpret_cast<qb::Qbf1Answer*>(key + qb::kQbf1Threads);
   QB_CUDA(cudaMemsetAsync(key, 0xff, key_bytes + sizeof(qb::Qbf1Answer), h->st));
   QB_CUDA(cudaEventRecord(h->ev[0], h->st));
@@ -1300,16 +1300,16 @@ int batch_run(qb_handle* h, const qb_problem* problems, const std::vector<int32_
   const size_t off_cand = ar.add(pre);  // last: the candidates' room reaches on from here
   // every device and pinned host allocation happens here
   QB_CUDA(B[1].ensure(off_cand + (size_t)cap * sizeof(qb::BatchCand)));
-  QB_CUDA(B[6].ensure((size_t)cap * sizeof(qb::ExactOut)));
-  QB_CUDA(B[7].ensure(std::max<uint64_t>(gtab_total, 4) * sizeof(float)));
-  QB_CUDA(B[8].ensure(std::max<uint64_t>(rec_total, 4) * sizeof(float)));
+  QB_CUDA(B[2].ensure((size_t)cap * sizeof(qb::ExactOut)));
+  QB_CUDA(B[3].ensure(std::max<uint64_t>(gtab_total, 4) * sizeof(float)));
+  QB_CUDA(B[4].ensure(std::max<uint64_t>(rec_total, 4) * sizeof(float)));
   QB_CUDA(h->hout.ensure(res_bytes));
   QB_CUDA(h->hstage.ensure(ar.size));
   char* dar = static_cast<char*>(B[1].p);
   char* har = static_cast<char*>(h->hstage.p);
   for (size_t k = 0; k < items.size(); ++k) {  // device addresses of the items' W and records
     items[k].W = static_cast<const double*>(B[0].p) + offs[k].first;
-    items[k].rec = static_cast<float*>(B[8].p) + offs[k].second;
+    items[k].rec = static_cast<float*>(B[4].p) + offs[k].second;
   }
   ar.fill(har);
   memset(har + off_res, 0xff, 2 * mb);
@@ -1326,7 +1326,7 @@ int batch_run(qb_handle* h, const qb_problem* problems, const std::vector<int32_
   const double* dW = static_cast<const double*>(B[0].p);
   const qb::BatchInst* dI = reinterpret_cast<const qb::BatchInst*>(dar + off_inst);
   qb::BatchCand* dC = reinterpret_cast<qb::BatchCand*>(dar + off_cand);
-  qb::ExactOut* dO = static_cast<qb::ExactOut*>(B[6].p);
+  qb::ExactOut* dO = static_cast<qb::ExactOut*>(B[2].p);
   qb::TcParams P{};
   size_t sm_tc = 0;
   if (!tcs.empty()) {
@@ -1341,8 +1341,6 @@ int batch_run(qb_handle* h, const qb_problem* problems, const std::vector<int32_
       sm_tc = std::max<size_t>(L.total, 120 * 1024) + 1024;
     }
   }
-  if (any_gray) {
-  }
   const unsigned key_blocks = (unsigned)std::min<int>((cap + 255) / 256, h->sm_count * 4);
 
   // the exact kernel's CTAs take candidates in turn: as many as run at once, if there are that many
@@ -1355,10 +1353,10 @@ int batch_run(qb_handle* h, const qb_problem* problems, const std::vector<int32_
     if (timed) QB_CUDA(cudaEventRecord(h->ev[0], st));
     if (any_gray) {
       qb::batch_gtab_kernel<<<(unsigned)gitems.size(), 256, sm_gtab, st>>>(
-          dI, reinterpret_cast<const qb::BatchItem*>(dar + off_git), dW, static_cast<float*>(B[7].p));
+          dI, reinterpret_cast<const qb::BatchItem*>(dar + off_git), dW, static_cast<float*>(B[3].p));
       qb::batch_gray_kernel<<<(unsigned)uitems.size(), qb::kGrayThreads, sm_gray, st>>>(
-          dI, reinterpret_cast<const qb::BatchItem*>(dar + off_uit), dW, static_cast<const float*>(B[7].p),
-          static_cast<float*>(B[8].p));
+          dI, reinterpret_cast<const qb::BatchItem*>(dar + off_uit), dW, static_cast<const float*>(B[3].p),
+          static_cast<float*>(B[4].p));
       h->kernels += 2;
     }
     if (!tcs.empty()) {
@@ -1374,7 +1372,7 @@ int batch_run(qb_handle* h, const qb_problem* problems, const std::vector<int32_
     if (timed) QB_CUDA(cudaEventRecord(h->ev[1], st));
     if (!gray_ids.empty()) {
       qb::batch_select_kernel<<<(unsigned)gray_ids.size(), 256, 0, st>>>(
-          dI, reinterpret_cast<const uint32_t*>(dar + off_gid), static_cast<const float*>(B[8].p), dC, ccount, cap,
+          dI, reinterpret_cast<const uint32_t*>(dar + off_gid), static_cast<const float*>(B[4].p), dC, ccount, cap,
           p1min, emin, kmin);
       ++h->kernels;
     }
@@ -1411,8 +1409,8 @@ int batch_run(qb_handle* h, const qb_problem* problems, const std::vector<int32_
       shape.offsets[i++] = off;
     i = 0;
     for (const void* a : {(const void*)Wall, (const void*)h->hstage.p, (const void*)h->hout.p, (const void*)h->own,
-                          (const void*)B[0].p, (const void*)B[1].p, (const void*)B[6].p, (const void*)B[7].p,
-                          (const void*)B[8].p})
+                          (const void*)B[0].p, (const void*)B[1].p, (const void*)B[2].p, (const void*)B[3].p,
+                          (const void*)B[4].p})
       shape.addresses[i++] = (uint64_t)(uintptr_t)a;
     const std::vector<uint64_t> key = qb::batch_graph_key(shape);
     if (!h->batch_graph || key != h->batch_graph_key) {

@@ -785,7 +785,7 @@ __global__ void __launch_bounds__(kTc2Threads, 1) tc_pair_kernel(const __grid_co
   float* EU = reinterpret_cast<float*>(tc_smem + L.eu_off);
   float* EY = reinterpret_cast<float*>(tc_smem + L.ey_off);
   float* Rs = reinterpret_cast<float*>(tc_smem + L.rs_off);          // per B stage: row terms of the block
-  float* Es = reinterpret_cast<float*>(tc_smem + L.es_off);          // per B stage: energy of low pattern 2 s + b
+  float* Es = reinterpret_cast<float*>(tc_smem + L.es_off);          // ring of kTc2EsRing blocks: energy of low pattern 2 s + b
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tc_smem + L.misc_off);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tc_smem + L.misc_off + 4);
   double* LO = reinterpret_cast<double*>(tc_smem + L.lo_off);
@@ -834,7 +834,7 @@ __global__ void __launch_bounds__(kTc2Threads, 1) tc_pair_kernel(const __grid_co
   }
   // A operands (constant, the same for every item), one per low pattern st: A[y][i] = y_i
   // (i < 7); the column term's digits (slots 8-10) 1, 2048, 32768; low t bit m (slots
-  // kLowSlot[m], kLowSlot[m] + 1, or 7 and 15) bit m of st times 1, 2048
+  // tc2_low_slot(m, 0) and (m, 1)) bit m of st times 1, 2048
   load_item(it_lo);
   for (int e = tid; e < NS * 128 * 2; e += kTc2Threads) {  // 8 columns (16 bytes) at a time
     const int st = e >> 8, y = (e >> 1) & 127, kh = e & 1;
@@ -1291,10 +1291,7 @@ inline int tc2_launch(const TcPlan& p, const float* gamma, float* rec, const dou
   Q.whi[0] = gamma[5];
   Q.whi[1] = gamma[6];
   Q.whi[2] = gamma[7];
-  if (p.u16) {
-    P.dmin = p.dmin;
-    tc2_u16_tables(gamma, p.dmin, &Q.tab);
-  }
+  if (p.u16) tc2_u16_tables(gamma, p.dmin, &Q.tab);
   const TcSmemLayout L = tc_layout(p.n);
   const size_t smem = p.u16 ? tc2_smem_bytes(p.n) : std::max<size_t>(L.total + kTcBStages * 128 * 4, 120 * 1024) + 1024;
   auto* kern = p.u16 ? tc_pair_kernel<false> : tc_pair_fp32_kernel;
