@@ -606,8 +606,9 @@ bool take_row(const Plan& P, const qb::ExactOut& row, qb::ExactOut* best) {
 // of the control block to the host.  The 16-bit pair kernel reduces its records' minimum itself,
 // so that a solve is three launches (four under QB_F1's rule) and one round trip; the whole call
 // at n = 20 .. 28 took 107 us with the scaling, threshold and final kernels and the clears on
-// their own (84 us without them), and 165 us with QB_F1's five round trips (94 us).  Returns -1 when the candidates overflow
-// the cap (the caller then takes the two-phase path with a larger cap).
+// their own (84 us without them), and 165 us with QB_F1's five round trips (94 us).  Returns -1
+// when the candidates overflow the cap (the caller then takes the two-phase path with a larger
+// cap).
 int solve_fused(qb_handle* h, const Plan& P, qb_result* r) {
   qb::SolveCtl* ctl = dev_ctl(h);
   const qb::ProblemDev pd{P.n, dev_W(h)};
@@ -1587,9 +1588,10 @@ int qb_prefix_minima(qb_handle* h, const qb_problem* p, int32_t prefix_bits, dou
     return QB_OK;
   }
   // few prefixes: each split over 2^sb CTAs (of at least 2^14 states) as long as all of them run
-  // at once, two per SM; more CTAs repeat the set-up, fewer leave SMs idle.  Measured for the
-  // whole call (us, the winner's thread walking again) at sb = 0 1 2 3 4 5: n = 27, A = 7 182 128 132 149 167 221; n = 24, A = 4
-  // 177 113 77 56 52 58; n = 23, A = 3 176 112 77 55 52 43; n = 30, A = 10 683 672 738 864
+  // at once, two per SM; more CTAs repeat the set-up, fewer leave SMs idle.  Measured for the whole
+  // call (us, uniform float Q) at sb = 0 1 2 ..: n = 28, A = 8 144 157 162 195; n = 27, A = 7 119 94
+  // 96 119 146; n = 26, A = 6 126 88 67 78 96; n = 25, A = 5 118 81 57 47 58 72; n = 24, A = 4 119 82
+  // 56 45 45 57; n = 22, A = 2 125 87 62 50 47 40 41 50
   int sb = 0;
   while (sb < B - 14 && (count << (sb + 1)) <= 2ull * (uint64_t)h->sm_count) ++sb;
   const uint64_t nout = count << sb;

@@ -16,12 +16,12 @@
 //
 // What bounds it: for one candidate record of 2^17 states in 16 parts (a 36-variable solve) the
 // latency of one CTA's steps -- W from L2, the base state's fields and the start tables (all
-// threads together), 32 energies, the CTA's minimum, one ordered sum: 10-12 us, against 29-54 us
-// when every thread summed its start and its best state's energy alone (n = 20 .. 37; 2^19-state
-// records of n = 40 158 -> 33 us).  Many states per CTA (2^19, qb_prefix_minima at n = 27): per
-// state one FP64 add and one FP64 compare with two selects, two CTAs per SM (128 registers);
-// 2^27 states 520 -> 69 us (105 when the winner's thread always walked again: seven of a CTA's
-// eight warps waited for it).  The 4096-problem batch's pass 2 1400 -> 507 us.
+// threads together), 32 energies, the CTA's minimum, one ordered sum: 15-18 us, against 29-54 us
+// when every thread summed its start and its best state's energy alone (n = 20 .. 37).  Many states
+// per CTA (2^19, qb_prefix_minima at n = 27): per state one FP64 add and one FP64 compare with two
+// selects, two CTAs per SM (128 registers); 2^27 states 520 -> 69 us.  Where nearly all states tie,
+// the second walk and the tie keys: 2^30 states of a zero matrix 2.0 ms, of a random one 0.46 ms.
+// The 4096-problem batch's pass 2 1400 -> 507 us.
 #pragma once
 #include <cstring>
 
