@@ -40,11 +40,9 @@ def test_prefix_minima(cuda_ok, n, A):
     assert [int(v) for v in got] == [int(v) for v in want]
 
 
-@pytest.mark.parametrize("n,form", [(16, "exact"), (20, "exact"), (20, "gray"), (20, "tc")])
-@pytest.mark.parametrize("rule", ["qbf", "natural", "qb_f1"])
+@pytest.mark.parametrize("n,form,rule", [(16, "exact", "qbf"), (16, "exact", "natural")] +
+                         [(20, form, rule) for form in ("exact", "gray", "tc") for rule in ("qbf", "natural", "qb_f1")])
 def test_solve(cuda_ok, n, form, rule):
-    if rule == "qb_f1" and n < 19:
-        pytest.skip("QB_F1's rule needs 19 variables")
     Q = _heavy(n, n + 1)
     E = _energies(Q)
     assert (E == E.min()).sum() == 1 and np.abs(Q).sum() < 2 ** 53
